@@ -375,7 +375,7 @@ _ref = None
 
 
 def build_reference_host():
-    if not os.path.isdir(REFERENCE_DIR):
+    if not os.path.exists(os.path.join(REFERENCE_DIR, "rtm_model.cu")):
         return False
     subprocess.run(["make", "-s", "-C", os.path.join(HERE, "ref"), "host", f"REF={REFERENCE_DIR}"], check=True)
     return os.path.exists(REF_HOST)
