@@ -131,18 +131,20 @@ struct rtm_session {
     TileRef *d_tiles_p = nullptr;    // tiles of the pressure kernels (whole padded grid)
     TileRef *d_tiles_r = nullptr;    // velocity tiles of the reconstruction region (interior + strips)
     TileRef *d_tiles_pr = nullptr;   // pressure tiles of the reconstruction region
-    // rows per tile (measured): 32 for the forward and receiver velocity kernels, 16 for the
-    // velocity reconstruction and the pressure kernels (forward and receiver pressure share
-    // one tile list; the pressure reconstruction has its own)
-    int bz_vel = 32, bz_vel_recon = 16, bz_pres = 16, bz_pres_recon = 16;
+    // merged lists of the backward pass: reconstruction pressure + receiver velocity; receiver
+    // pressure + the next step's reconstruction velocity
+    TileRef *d_tiles_m[2] = {nullptr, nullptr};
+    // rows per tile without the tuner (forward and receiver kernels of a field share one tile list;
+    // the reconstruction kernels have their own)
+    int bz_vel = 16, bz_vel_recon = 16, bz_pres = 16, bz_pres_recon = 16;
     // kernel form per family (forward/receiver velocity, reconstruction velocity, forward/receiver
-    // pressure, reconstruction pressure): four columns by U rows per thread (rtm_stencil_v.cu)
-    // or one column per thread (rtm_stencil.cu); the results are the same bits.  Chosen by the
-    // tuner with the tile heights; without it the measured defaults (one column per thread for
-    // the full-grid kernels, four columns for the reconstruction), or all of one form with
-    // RTM_B200_KERNELS=scalar|vector.
-    bool vec[4] = {false, true, false, true};
+    // pressure, reconstruction pressure): the pipelined one (rtm_pipe.cu) or one tile per block with
+    // one column per thread (rtm_stencil.cu), by RTM_B200_KERNELS=vector|scalar
+    bool vec[4] = {true, true, true, true};
     bool forms_fixed = false;
+    // backward pass in two merged launches per step (chosen by the tuner; needs every family in the
+    // pipelined form at one tile height)
+    bool merge = true;
     bool tune = true;                // choose the tile heights per launch shape by timing them
     // whole-step kernel (rtm_step.cu): velocity and pressure of a step in one launch over
     // tz_step-row tiles, two buffers per field, four descriptor tables (which buffer is
@@ -155,12 +157,14 @@ struct rtm_session {
     long long pass_wait_ns = 2000000000LL;   // bound on one wait (RTM_B200_PASS_WAIT_US)
     int *d_per_shot = nullptr;               // [6][B]: tiles per shot, source pass lists then backward lists
     unsigned *d_queue = nullptr, *d_done = nullptr;   // pass queue counter; [4][B] completion counters
+    unsigned *d_pipe_queue = nullptr;        // the pipelined kernels' two tile counters
+    int pipe_sel = 0;                        // the one the next pipelined launch takes its tiles from
     unsigned *d_trace = nullptr;             // the item each persistent block took last
     int trace_len = 0;
     void *d_fin = nullptr;
     void *d_tmaps = nullptr;         // B x RTM_TMAP_COUNT tensor maps (rebuilt for every batch)
     int *d_err = nullptr;            // kernel error flag (bounded waits that gave up)
-    int *d_counts = nullptr;         // tile counts of the batch's four lists (fixed-grid launches)
+    int *d_counts = nullptr;         // tile counts of the batch's lists (fixed-grid launches)
     int max_tiles = 0;
     std::map<std::string, rtm::KernelTiming> timing;
     int launches = 0;
@@ -367,8 +371,15 @@ static int acc_bytes(const rtm_options &o)
     return o.accum_fp64 == RTM_ACC_FP64 || o.accum_fp64 == RTM_ACC_KAHAN ? 8 : 4;
 }
 
-static size_t slot_bytes(const rtm_survey &s, const rtm_options &o, int pitch, int Z, int strip_len, int nxi, int nzi,
-                         bool fused)
+// Tiles of one X x Z shot at the shortest tile height the tuner or the environment may choose.
+static int max_shot_tiles(int X, int Z)
+{
+    const int bz_min = 8;
+    return ((X + RTM_BX - 1) / RTM_BX + 1) * ((Z + bz_min - 1) / bz_min + 1);
+}
+
+static size_t slot_bytes(const rtm_survey &s, const rtm_options &o, int X, int pitch, int Z, int strip_len, int nxi,
+                         int nzi, bool fused)
 {
     size_t field = (size_t)pitch * Z * sizeof(float) + 256;
     size_t b = (fused ? 16 : 10) * field;
@@ -380,6 +391,7 @@ static size_t slot_bytes(const rtm_survey &s, const rtm_options &o, int pitch, i
     b += 2 * ((size_t)pitch * Z * acc_bytes(o) + 256);   // g1, illum on the padded grid
     if (o.accum_fp64 == RTM_ACC_FP64_BLOCKED) b += 2 * ((size_t)pitch * Z * 8 + 256);   // their fp64 totals
     if (o.extra_images) b += 4 * ((size_t)pitch * Z * (o.accum_fp64 ? 8 : 4) + 256) + 2 * field;
+    b += 8 * sizeof(TileRef) * (size_t)max_shot_tiles(X, Z) + RTM_TMAP_COUNT * RTM_TMAP_BYTES;   // tables
     (void)nxi;
     (void)nzi;
     return b;
@@ -467,7 +479,7 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
         if ((e = std::getenv("RTM_B200_PERSIST")) && *e) ss->persist = std::atoi(e) != 0 && !ss->fused;
         if ((e = std::getenv("RTM_B200_PASS_WAIT_US")) && *e) ss->pass_wait_ns = std::atoll(e) * 1000LL;
     }
-    size_t per_slot = slot_bytes(s, o, big.pitch, big.Z, big.strip_len, big.nxi, big.nzi, ss->fused);
+    size_t per_slot = slot_bytes(s, o, big.X, big.pitch, big.Z, big.strip_len, big.nxi, big.nzi, ss->fused);
     size_t fixed = model_bytes + shot_bytes_total + (o.extra_images ? 11 : 4) * ((size_t)s.nx * s.nz * 8 + 256) + (size_t)s.nt * 4 + 4096 +
                    (size_t)(64 << 20);
     size_t budget = (size_t)(free_b * 0.92);
@@ -669,22 +681,23 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
         }
     }
     CK(cudaMemsetAsync(ss->d_err, 0, 8 * sizeof(int), ss->stream));
-    // tile tables sized for the shortest tile height the tuner or the environment may choose
-    const int bz_min = 8;
-    int tiles_per_shot = ((big.X + RTM_BX - 1) / RTM_BX + 1) * ((big.Z + bz_min - 1) / bz_min + 1);
-    ss->max_tiles = tiles_per_shot * B;
+    ss->max_tiles = max_shot_tiles(big.X, big.Z) * B;
     ss->d_tiles = (TileRef *)ss->arena.take(sizeof(TileRef) * ss->max_tiles);
     ss->d_tiles_p = (TileRef *)ss->arena.take(sizeof(TileRef) * ss->max_tiles);
     ss->d_tiles_r = (TileRef *)ss->arena.take(sizeof(TileRef) * ss->max_tiles);
     ss->d_tiles_pr = (TileRef *)ss->arena.take(sizeof(TileRef) * ss->max_tiles);
+    for (TileRef *&m : ss->d_tiles_m)
+        if (!(m = (TileRef *)ss->arena.take(sizeof(TileRef) * 2 * (size_t)ss->max_tiles)))
+            return fail(RTM_ERR_NOMEM, "device arena exhausted (tables)");
     ss->d_fin = ss->arena.take(finalize_shot_size() * B);
-    ss->d_counts = (int *)ss->arena.take(4 * sizeof(int));
+    ss->d_counts = (int *)ss->arena.take(6 * sizeof(int));
     ss->d_per_shot = (int *)ss->arena.take(6 * sizeof(int) * B);
     ss->d_queue = (unsigned *)ss->arena.take(2 * sizeof(unsigned));
+    ss->d_pipe_queue = (unsigned *)ss->arena.take(2 * sizeof(unsigned));
     ss->d_done = (unsigned *)ss->arena.take(4 * sizeof(unsigned) * B);
     ss->trace_len = 148 * 16;
     ss->d_trace = (unsigned *)ss->arena.take(sizeof(unsigned) * ss->trace_len);
-    if (!ss->d_counts || !ss->d_per_shot || !ss->d_queue || !ss->d_done)
+    if (!ss->d_counts || !ss->d_per_shot || !ss->d_queue || !ss->d_done || !ss->d_pipe_queue)
         return fail(RTM_ERR_NOMEM, "device arena exhausted (tables)");
     if (!ss->d_shots || !ss->d_tiles || !ss->d_tiles_p || !ss->d_tiles_r || !ss->d_tiles_pr || !ss->d_fin)
         return fail(RTM_ERR_NOMEM, "device arena exhausted (tables)");
@@ -756,6 +769,23 @@ static void timing_end(rtm_session *ss, cudaEvent_t ev)
     if (ev) cudaEventRecord(ev, ss->stream);
 }
 
+// A pipelined launch; the two tile counters alternate.
+static void pipe_step(rtm_session *ss, int pm, int vm, int bz, const StepArgs &a0, int ntiles, int record)
+{
+    StepArgs a = a0;
+    a.queue = ss->d_pipe_queue;
+    a.qsel = ss->pipe_sel;
+    ss->pipe_sel ^= 1;
+    launch_pipe(pm, vm, bz, a, ntiles, record, ss->stream);
+}
+// Before the first pipelined launch of a pass (inside the captured part of a graph): both
+// counters zero.
+static void pipe_reset(rtm_session *ss)
+{
+    cudaMemsetAsync(ss->d_pipe_queue, 0, 2 * sizeof(unsigned), ss->stream);
+    ss->pipe_sel = 0;
+}
+
 // Batch state shared by the phases of one batch.
 struct BatchRun {
     int k0 = 0, n = 0, ntiles = 0, ntiles_p = 0, ntiles_r = 0, ntiles_pr = 0, maxrec = 0, max_strip_len = 0;
@@ -767,7 +797,11 @@ struct BatchRun {
     // rounded up to four significant bits, so that one captured graph serves batches whose
     // windows differ a little; likewise the strip kernels' and the other imaging conditions'
     // extents
-    int grid[4] = {0, 0, 0, 0};
+    int grid[6] = {0, 0, 0, 0, 0, 0};
+    // backward pass in merged launches (d_tiles_m): every family in the pipelined form at one
+    // tile height, and no kernel that reads the reconstructed velocities between them
+    bool merged = false, heavy_first = false;
+    int nmerged[2] = {0, 0};
     int strip_grid = 0, ex_nxi = 0, ex_nzi = 0;
 };
 
@@ -833,12 +867,19 @@ static void shot_tiles(const rtm_session *ss, const ShotState &sh, int j, bool f
     const int zr0 = s.npml - RTM_RADIUS, zr1 = sh.Z - s.npml + RTM_RADIUS;
     // velocity tiles: interior when every column lies in [npml, X-npml-1) and every row in
     // [npml, Z-npml-1), where the velocity damping is 1 and no strip lies
+    // what a tile that is not interior holds (RTM_TILE_*; the pipelined kernels test for it)
+    auto bits = [&](bool band, int x0, bool src, bool rec) {
+        const bool edge = x0 < RTM_RADIUS || x0 + RTM_BX > sh.X - RTM_RADIUS;
+        return (band ? RTM_TILE_XBAND : 0) | (edge ? RTM_TILE_XEDGE : 0) | (src ? RTM_TILE_SRC : 0) |
+               (rec ? RTM_TILE_REC : 0);
+    };
     auto add_tiles = [&](std::vector<TileRef> &v, int bz, int xa, int xb, int za, int zb) {
         for (int z0 = za; z0 < zb; z0 += bz)
             for (int x0 = xa; x0 < xb; x0 += RTM_BX) {
                 const bool inside = x0 >= s.npml && x0 + RTM_BX <= sh.X - s.npml - 1 && z0 >= s.npml &&
                                     z0 + bz <= sh.Z - s.npml - 1;
-                v.push_back({j, x0, z0, (fast && inside) ? 1 : 0});
+                const bool band = x0 < s.npml || x0 + RTM_BX > sh.X - s.npml - 1;
+                v.push_back({j, x0, z0, (fast && inside) ? 1 : bits(band, x0, false, false)});
             }
     };
     if (ss->fused) {
@@ -870,7 +911,12 @@ static void shot_tiles(const rtm_session *ss, const ShotState &sh, int j, bool f
             const bool inside = x0 >= s.npml && x1 <= sh.X - s.npml && z0 >= s.npml && z1 <= sh.Z - s.npml;
             const bool src = x0 < sh.sbx0 + sh.sbnx && sh.sbx0 < x1 && z0 < sh.sbz0 + sh.sbnz && sh.sbz0 < z1;
             const bool rec = sh.g.rz >= z0 && sh.g.rz < z1 && x0 < sh.g.rx0 + sh.g.nrec && sh.g.rx0 < x1;
-            tiles_p.push_back({j, x0, z0, (fast && inside && !src && !rec) ? 1 : 0});
+            const bool band = x0 < s.npml || x1 > sh.X - s.npml;
+            const bool img = x0 < sh.X - s.npml && x1 > s.npml && z0 < sh.Z - s.npml && z1 > s.npml;
+            tiles_p.push_back({j, x0, z0, (fast && inside && !src && !rec)
+                                              ? 1
+                                              : bits(band, x0, src, rec) | (inside ? 0 : RTM_TILE_BAND) |
+                                                    (img ? RTM_TILE_IMG : 0)});
         }
     if (!ss->fused) add_tiles(tiles_r, ss->bz_vel_recon, xr0, xr1, zr0, zr1);
     // reconstruction pressure tiles: interior when inside the pressure interior with no
@@ -880,7 +926,8 @@ static void shot_tiles(const rtm_session *ss, const ShotState &sh, int j, bool f
             const int x1 = x0 + RTM_BX, z1 = z0 + ss->bz_pres_recon;
             const bool inside = x0 >= s.npml && x1 <= sh.X - s.npml && z0 >= s.npml && z1 <= sh.Z - s.npml;
             const bool src = x0 < sh.sbx0 + sh.sbnx && sh.sbx0 < x1 && z0 < sh.sbz0 + sh.sbnz && sh.sbz0 < z1;
-            tiles_pr.push_back({j, x0, z0, (fast && inside && !src) ? 1 : 0});
+            const bool band = x0 < s.npml || x1 > sh.X - s.npml;
+            tiles_pr.push_back({j, x0, z0, (fast && inside && !src) ? 1 : bits(band, x0, src, false)});
         }
 }
 
@@ -926,22 +973,36 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
         d.vp2_b = sh.mb.vp2;
         // tensor maps of the fields the stencil kernels stage, for this shot's row pitch
         {
-            const int vh = ss->bz_vel + RTM_STAGE_ZEXTRA_VEL, ph = ss->bz_pres + RTM_STAGE_ZEXTRA_PRES;
-            const int vhr = ss->bz_vel_recon + RTM_STAGE_ZEXTRA_VEL, phr = ss->bz_pres_recon + RTM_STAGE_ZEXTRA_PRES;
+            // (the pipelined form stages the 19 rows its derivatives reach beyond a tile)
+            const int vh = ss->bz_vel + (ss->vec[0] ? 19 : RTM_STAGE_ZEXTRA_VEL);
+            const int vhr = ss->bz_vel_recon + (ss->vec[1] ? 19 : RTM_STAGE_ZEXTRA_VEL);
+            const int ph = ss->bz_pres + (ss->vec[2] ? 19 : RTM_STAGE_ZEXTRA_PRES);
+            const int phr = ss->bz_pres_recon + (ss->vec[3] ? 19 : RTM_STAGE_ZEXTRA_PRES);
             // whole-step kernel: p of both buffers of each wavefield (placeholders when off)
             const int sw = RTM_BX + 48, sh_ = ss->tz_step + 38;
             const WaveDev &A1 = ss->fused ? sl.a2 : sl.a, &B1 = ss->fused ? sl.b2 : sl.b;
-            const int tz = ss->tz_step;
+            const int tz = ss->tz_step, aw = acc_bytes(o) / 4;   // (words per accumulator)
             struct { float *f; int w, h; } m[RTM_TMAP_COUNT] = {
                 {sl.a.p, RTM_STAGE_W, vh}, {sl.a.vx, RTM_STAGE_W, ss->bz_pres}, {sl.a.vz, RTM_BX, ph},
                 {sl.b.p, RTM_STAGE_W, vh}, {sl.b.vx, RTM_STAGE_W, ss->bz_pres}, {sl.b.vz, RTM_BX, ph},
                 {sl.a.p, RTM_STAGE_W, vhr}, {sl.a.p, sw, sh_}, {A1.p, sw, sh_}, {sl.b.p, sw, sh_}, {B1.p, sw, sh_},
                 {sl.a.vx, RTM_STAGE_W, tz}, {A1.vx, RTM_STAGE_W, tz}, {sl.b.vx, RTM_STAGE_W, tz}, {B1.vx, RTM_STAGE_W, tz},
                 {sl.a.vz, RTM_BX, tz + 20}, {A1.vz, RTM_BX, tz + 20}, {sl.b.vz, RTM_BX, tz + 20}, {B1.vz, RTM_BX, tz + 20},
-                {sl.a.vx, RTM_STAGE_W, ss->bz_pres_recon}, {sl.a.vz, RTM_BX, phr}};
+                {sl.a.vx, RTM_STAGE_W, ss->bz_pres_recon}, {sl.a.vz, RTM_BX, phr},
+                {sh.mf.inv_rho, RTM_BX, ss->bz_vel}, {sh.mb.inv_rho, RTM_BX, ss->bz_vel},
+                {sl.a.vx, RTM_BX, ss->bz_vel}, {sl.a.vz, RTM_BX, ss->bz_vel},
+                {sl.b.vx, RTM_BX, ss->bz_vel}, {sl.b.vz, RTM_BX, ss->bz_vel},
+                {sh.mb.inv_rho, RTM_BX, ss->bz_vel_recon}, {sl.a.vx, RTM_BX, ss->bz_vel_recon},
+                {sl.a.vz, RTM_BX, ss->bz_vel_recon}, {sh.mf.kappa, RTM_BX, ss->bz_pres},
+                {sh.mb.kappa, RTM_BX, ss->bz_pres}, {sl.a.p, RTM_BX, ss->bz_pres}, {sl.b.p, RTM_BX, ss->bz_pres},
+                {sh.mb.kappa, RTM_BX, ss->bz_pres_recon}, {sl.a.p, RTM_BX, ss->bz_pres_recon},
+                {sl.a.sx, RTM_BX, ss->bz_pres}, {sl.a.sz, RTM_BX, ss->bz_pres}, {sl.b.sx, RTM_BX, ss->bz_pres},
+                {sl.b.sz, RTM_BX, ss->bz_pres}, {(float *)sl.g1, aw * RTM_BX, ss->bz_pres},
+                {(float *)sl.illum, aw * RTM_BX, ss->bz_pres}};
             for (int t = 0; t < RTM_TMAP_COUNT; t++) {
                 CUtensorMap cm;
-                int rc = encode_field_map(&cm, m[t].f, sh.pitch, sh.Z, m[t].w, m[t].h);
+                const int pw = t == RTM_TMAP_G1 || t == RTM_TMAP_ILLUM ? aw : 1;
+                int rc = encode_field_map(&cm, m[t].f, pw * sh.pitch, sh.Z, m[t].w, m[t].h);
                 if (rc) return rc;
                 std::memcpy(&maps[((size_t)j * RTM_TMAP_COUNT + t) * RTM_TMAP_BYTES], &cm, RTM_TMAP_BYTES);
             }
@@ -978,13 +1039,48 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
                     return a.z0 != b.z0 ? a.z0 < b.z0 : a.x0 < b.x0;
                 });
     }
+    {
+        // a batch whose fields stay in L2 (about 10 arrays per shot): the tiles with PML, source,
+        // receiver or strip cells first, since they take two to three times as long as interior
+        // ones and the blocks take tiles as they finish; larger batches keep the tiles in field
+        // order, for the L2 reuse of halo rows between neighbours
+        size_t bytes = 0;
+        for (int j = 0; j < n; j++) bytes += (size_t)10 * 4 * ss->shots[k0 + j].pitch * ss->shots[k0 + j].Z;
+        br.heavy_first = bytes <= ((size_t)160 << 20);
+        if (br.heavy_first)
+            for (std::vector<TileRef> *v : {&tiles, &tiles_p, &tiles_r, &tiles_pr})
+                std::stable_partition(v->begin(), v->end(), [](const TileRef &t) { return !(t.interior & 1); });
+    }
     br.ntiles = (int)tiles.size();
     br.ntiles_p = (int)tiles_p.size();
     br.ntiles_r = (int)tiles_r.size();
     br.ntiles_pr = (int)tiles_pr.size();
     if (std::max(std::max(br.ntiles, br.ntiles_p), std::max(br.ntiles_r, br.ntiles_pr)) > ss->max_tiles)
         return fail(RTM_ERR_ARG, "tile table overflow");
-    const int counts[4] = {br.ntiles, br.ntiles_p, br.ntiles_r, br.ntiles_pr};
+    br.merged = ss->merge && ss->vec[0] && ss->vec[1] && ss->vec[2] && ss->vec[3] && ss->bz_vel == ss->bz_vel_recon &&
+                ss->bz_vel == ss->bz_pres && ss->bz_vel == ss->bz_pres_recon && !ss->fused && !o.extra_images;
+    if (br.merged) {
+        // both kinds in the order of their rows, so that tiles of one region run close together
+        // (the receiver pressure's imaging and the reconstruction velocity read the same
+        // reconstructed pressure)
+        const std::vector<TileRef> *pv[2][2] = {{&tiles_pr, &tiles}, {&tiles_p, &tiles_r}};
+        for (int m = 0; m < 2; m++) {
+            std::vector<TileRef> v = *pv[m][0];
+            for (TileRef t : *pv[m][1]) {
+                t.interior |= RTM_TILE_VEL;
+                v.push_back(t);
+            }
+            if (br.heavy_first)
+                std::stable_partition(v.begin(), v.end(), [](const TileRef &t) { return !(t.interior & 1); });
+            else
+                std::stable_sort(v.begin(), v.end(), [](const TileRef &a, const TileRef &b) {
+                    return a.shot != b.shot ? a.shot < b.shot : a.z0 < b.z0;
+                });
+            br.nmerged[m] = (int)v.size();
+            CK(cudaMemcpyAsync(ss->d_tiles_m[m], v.data(), sizeof(TileRef) * v.size(), cudaMemcpyHostToDevice, st));
+        }
+    }
+    const int counts[6] = {br.ntiles, br.ntiles_p, br.ntiles_r, br.ntiles_pr, br.nmerged[0], br.nmerged[1]};
     CK(cudaMemcpyAsync(ss->d_counts, counts, sizeof(counts), cudaMemcpyHostToDevice, st));
     {   // tiles per shot: source pass lists (velocity, pressure), backward lists (reconstruction
         // velocity and pressure, receiver velocity and pressure)
@@ -995,7 +1091,7 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
         CK(cudaMemcpyAsync(ss->d_per_shot, per.data(), sizeof(int) * per.size(), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));   // the host vector goes out of scope
     }
-    for (int L = 0; L < 4; L++) br.grid[L] = counts[L];
+    for (int L = 0; L < 6; L++) br.grid[L] = counts[L];
     br.strip_grid = br.max_strip_len;
     for (int j = 0; j < n; j++) {
         br.ex_nxi = std::max(br.ex_nxi, ss->shots[k0 + j].nxi);
@@ -1010,7 +1106,7 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
             while ((v >> e) >= 16) e++;
             return ((v + (1 << e) - 1) >> e) << e;
         };
-        for (int l = 0; l < 4; l++) br.grid[l] = bucket(counts[l]);
+        for (int l = 0; l < 6; l++) br.grid[l] = bucket(counts[l]);
         br.strip_grid = bucket(br.strip_grid);
         br.ex_nxi = bucket(br.ex_nxi);
         br.ex_nzi = bucket(br.ex_nzi);
@@ -1021,6 +1117,7 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
         br.hd[j].bn = sl.b2;
     }
     br.pa = br.pb = 0;
+    pipe_reset(ss);
     if (int rc = upload_tables(ss, br)) return rc;
     CK(cudaMemcpyAsync(ss->d_tmaps, maps.data(), maps.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ss->d_tiles, tiles.data(), sizeof(TileRef) * br.ntiles, cudaMemcpyHostToDevice, st));
@@ -1033,7 +1130,10 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
     a.tiles = ss->d_tiles;
     a.wavelet = ss->wavelet;
     a.coef = ss->coef;
-    for (int i = 0; i < 10; i++) a.c10[i] = ss->coef_host[90 + i];
+    for (int i = 0; i < 10; i++) {
+        a.c10[i] = ss->coef_host[90 + i];
+        a.c2[i] = make_float2(a.c10[i], a.c10[i]);
+    }
     a.dt = s.dt;
     a.dtx = s.dt / s.dx;   // rtm_model.cu:73-74
     a.dtz = s.dt / s.dz;
@@ -1064,12 +1164,12 @@ static int form_bits(const rtm_session *ss)
 // Stencil launches in the session's kernel form.
 static void vel_step(rtm_session *ss, int mode, int bz, const StepArgs &a, int ntiles)
 {
-    if (ss->vec[mode == RTM_WAVE_RECON ? 1 : 0]) launch_vel4(mode, bz, a, ntiles, ss->stream);
+    if (ss->vec[mode == RTM_WAVE_RECON ? 1 : 0]) pipe_step(ss, -1, mode, bz, a, ntiles, 0);
     else launch_vel(mode, bz, a, ntiles, ss->stream);
 }
 static void pres_step(rtm_session *ss, int mode, int bz, const StepArgs &a, int ntiles, int record)
 {
-    if (ss->vec[mode == RTM_WAVE_RECON ? 3 : 2]) launch_pres4(mode, bz, a, ntiles, record, ss->stream);
+    if (ss->vec[mode == RTM_WAVE_RECON ? 3 : 2]) pipe_step(ss, mode, -1, bz, a, ntiles, record);
     else launch_pres(mode, bz, a, ntiles, record, ss->stream);
 }
 
@@ -1214,7 +1314,11 @@ static int batch_forward(rtm_session *ss, BatchRun &br, int nsteps, bool save, b
     const int ntsnap = ss->nsnap ? (int)(o.tsnap / ss->s.dt) : 0;
     if (ntsnap) CK(cudaMemsetAsync(ss->d_absmax, 0, sizeof(unsigned) * ss->nsnap * ss->B, st));
     nvtxRangePushA(record && !save ? "rtm: modelling pass" : "rtm: source pass");
+    // the pipelined kernels save their strip cells themselves
+    const bool own_save = save && !ss->fused && !ss->persist && ss->vec[0] && ss->vec[2];
+    a.save = own_save;
     auto loop = [&] {
+        pipe_reset(ss);
         for (int it = 0; it < nsteps; it++) {
             a.it = it;
             a.ring = it % kRing;
@@ -1244,7 +1348,7 @@ static int batch_forward(rtm_session *ss, BatchRun &br, int nsteps, bool save, b
                 timing_end(ss, e);
                 ss->launches += 1;
             }
-            if (save) {
+            if (save && !own_save) {
                 timing_begin(ss, "strip_save", it, &e);
                 launch_strip_save(table(ss, br), br.n, br.strip_grid, it, a.ring, o.strip_precision, st);
                 timing_end(ss, e);
@@ -1333,6 +1437,7 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
     }
     if (int rc = upload_tables(ss, br)) return rc;
     a.gather_prec = o.gather_precision;
+    a.save = 0;
     // ps = final forward p; vxs = vzs = 0 (rtm_model.cu:367-372); the receiver wavefield
     // starts from rest with the last gather sample injected (:410)
     for (int j = 0; j < n; j++) {
@@ -1373,6 +1478,16 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
         ss->launches++;
     };
     auto loop = [&] {
+        pipe_reset(ss);
+        if (br.merged) {   // the first step's reconstruction velocity
+            cudaEvent_t e;
+            a.it = s.nt - 2;
+            timing_begin(ss, "vel_recon", 7, &e);
+            a.tiles = ss->d_tiles_r;
+            vel_step(ss, RTM_WAVE_RECON, ss->bz_vel_recon, a, list_grid(ss, br, a, 2));
+            timing_end(ss, e);
+            ss->launches++;
+        }
         for (int it = s.nt - 2; it >= 0; it--) {
             a.it = it;
             cudaEvent_t e;
@@ -1406,6 +1521,28 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
                                        s.dz, s.dt, st);
                     ss->launches++;
                 }
+                continue;
+            }
+            if (br.merged) {
+                // reconstruction pressure and receiver velocity of this step, then receiver
+                // pressure with imaging and the reconstruction velocity of the next: the kinds of
+                // a launch read and write different fields (both kinds of the second read the
+                // reconstructed pressure)
+                timing_begin(ss, "recon_recv", it, &e);
+                a.tiles = ss->d_tiles_m[0];
+                pipe_step(ss, RTM_WAVE_RECON, RTM_WAVE_RECEIVER, ss->bz_vel, a, list_grid(ss, br, a, 4), 0);
+                timing_end(ss, e);
+                timing_begin(ss, "recv_recon", it, &e);
+                if (it > 0) {
+                    a.tiles = ss->d_tiles_m[1];
+                    pipe_step(ss, RTM_WAVE_RECEIVER, RTM_WAVE_RECON, ss->bz_vel, a, list_grid(ss, br, a, 5), 0);
+                } else {
+                    launch_pres_tiles(ss, br, RTM_WAVE_RECEIVER, 0);
+                    ss->launches--;
+                }
+                timing_end(ss, e);
+                ss->launches += 2;
+                flush_images(it);
                 continue;
             }
             timing_begin(ss, "vel_recon", it, &e);
@@ -1445,8 +1582,8 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
     } else {
         const int pa0 = br.pa, pb0 = br.pb;
         int rc = run_pass(ss, {1, n, br.grid[0], br.grid[1], br.grid[2], br.grid[3], br.ex_nxi, br.ex_nzi,
-                               a.gather_prec, ss->bz_vel, ss->bz_vel_recon, ss->bz_pres, ss->bz_pres_recon,
-                               form_bits(ss), ss->fused, ss->tz_step, pa0, pb0}, loop);
+                               br.grid[4], br.grid[5], a.gather_prec, ss->bz_vel, ss->bz_vel_recon, ss->bz_pres, ss->bz_pres_recon,
+                               form_bits(ss), br.merged, ss->fused, ss->tz_step, pa0, pb0}, loop);
         if (!rc && ss->fused && ss->o.use_graph) {   // a replayed graph swaps as the captured loop did
             br.pa = pa0 ^ ((s.nt - 1) & 1);
             br.pb = pb0 ^ ((s.nt - 1) & 1);
@@ -1488,21 +1625,21 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
     return RTM_OK;
 }
 
-// ---- tile-height and kernel-form tuner ------------------------------------------------
-// The split stencil kernels take 8-, 16- or 32-row tiles in two forms (one column per thread;
-// four columns by U rows per thread); which is fastest depends on the grid (partial tiles, the
-// share of PML-band and edge tiles), on the shots per launch (blocks to fill 148 SMs) and on
-// the kernel.  Before the first batch of a launch shape, every (height, form) is timed on that
-// batch's own buffers: two untimed and four timed source-pass steps (velocity and pressure)
-// and backward steps (reconstruction and receiver pass) with CUDA events per kernel, no strips
-// saved.  Forward/receiver velocity, reconstruction velocity and reconstruction pressure each
-// keep their fastest pair; the forward and receiver pressure kernels share one height (one
-// tile list), each taking its faster form at it.  The batch is set up again afterwards, so
-// the trial steps leave nothing behind; heights and forms do not change the results (tested
-// bit for bit).  Choices are kept per process by launch shape and, with
-// RTM_B200_TUNE_CACHE=<file>, in that file ("key vel vel_recon pres pres_recon forms" lines,
-// forms a bit set of vel, vel_recon, pres, pres_recon) across processes.  The whole-step kernel's tile
-// height is chosen the same way (tune_step_height).
+// ---- tuner --------------------------------------------------------------------------
+// The split stencil kernels take 8-, 16- or 32-row tiles, and the backward pass runs in four
+// launches per step or in two merged ones; which is fastest depends on the grid (partial tiles,
+// the share of PML-band and edge tiles), on the shots per launch (tiles to fill 148 SMs) and on
+// the kernel.  Before the first batch of a launch shape, on that batch's own buffers: every
+// height is timed per kernel (two untimed and four timed source-pass and backward steps, no
+// strips saved), which gives each family its fastest one: forward/receiver velocity (one tile
+// list), reconstruction velocity, forward/receiver pressure (one tile list), reconstruction
+// pressure.  Then whole steps are timed back to back for that choice in separate launches and
+// for merged launches at 8 and 16 rows (merging needs one height), and the fastest plan is kept.
+// The batch is set up again afterwards, so the trial steps leave nothing behind; plans do not
+// change the results (tested bit for bit).  Choices are kept per process by launch shape and,
+// with RTM_B200_TUNE_CACHE=<file>, in that file ("key vel vel_recon pres pres_recon plan" lines,
+// plan a bit set: forms of vel, vel_recon, pres, pres_recon, then 16 for merged launches) across
+// processes.  The whole-step kernel's tile height is chosen the same way (tune_step_height).
 namespace {
 std::mutex g_tune_mu;
 std::map<std::string, std::array<int, 5>> g_tune;
@@ -1515,7 +1652,7 @@ static std::string tune_key(rtm_session *ss, int k0, int n)
     for (int j = 0; j < n; j++) xmax = std::max(xmax, ss->shots[k0 + j].X);
     char b[200];
     std::snprintf(b, sizeof b, "%s/X%d/Z%d/npml%d/n%d/strip%d/gather%d/acc%d/extra%d/mode%d",
-                  ss->fused ? "step" : ss->forms_fixed ? (ss->vec[0] ? "vector" : "scalar") : "split",
+                  ss->fused ? "step" : ss->vec[0] ? "pipe" : "scalar",
                   xmax, ss->shots[k0].Z, ss->s.npml, n, ss->o.strip_precision, ss->o.gather_precision, ss->o.accum_fp64,
                   ss->o.extra_images, ss->s.mode);
     return b;
@@ -1614,16 +1751,13 @@ static int tune_heights(rtm_session *ss, int k0, int n)
             ss->bz_pres = it->second[2];
             ss->bz_pres_recon = it->second[3];
             for (int f = 0; f < 4; f++) ss->vec[f] = (it->second[4] >> f) & 1;
+            ss->merge = (it->second[4] & 16) != 0;
             return RTM_OK;
         }
     }
     if (ss->fused) return tune_step_height(ss, k0, n, key, path);
-    // candidates: tile height x kernel form (both forms unless RTM_B200_KERNELS fixes one)
-    std::vector<std::pair<int, int>> cand;   // (bz, vector form)
-    for (int bz : {8, 16, 32})
-        for (int f = 0; f < 2; f++)
-            if (!ss->forms_fixed || f == (ss->vec[0] ? 1 : 0)) cand.push_back({bz, f});
-    const int nc = (int)cand.size();
+    const int cand[3] = {8, 16, 32}, nc = 3;   // tile heights
+    ss->merge = false;
     const char *names[6] = {"vel_fwd", "pres_fwd", "vel_recon", "pres_recon", "vel_recv", "pres_recv"};
     std::vector<std::array<double, 6>> ms(nc, std::array<double, 6>{});
     cudaEvent_t ev[2][6][4];
@@ -1634,8 +1768,7 @@ static int tune_heights(rtm_session *ss, int k0, int n)
     int rc = RTM_OK;
     const int steps = 6, warm = 2;
     for (int c = 0; c < nc && rc == RTM_OK; c++) {
-        ss->bz_vel = ss->bz_vel_recon = ss->bz_pres = ss->bz_pres_recon = cand[c].first;
-        for (bool &v : ss->vec) v = cand[c].second != 0;
+        ss->bz_vel = ss->bz_vel_recon = ss->bz_pres = ss->bz_pres_recon = cand[c];
         BatchRun br;
         if ((rc = batch_setup(ss, k0, n, br))) break;
         StepArgs a = br.a;
@@ -1670,34 +1803,99 @@ static int tune_heights(rtm_session *ss, int k0, int n)
             for (auto &e : b) cudaEventDestroy(e);
     if (rc) return rc;
     if ((rc = check_kernel_flag(ss))) return rc;
-    // the fastest (height, form) of each family, the forward and receiver kernels of a field
-    // together (they share a tile list and a form)
+    // the fastest height of each family, the forward and receiver kernels of a field together (they
+    // share a tile list)
     auto argmin = [&](auto cost) {
         int bi = 0;
         for (int c = 1; c < nc; c++)
             if (cost(c) < cost(bi)) bi = c;
-        return bi;
+        return cand[bi];
     };
-    const int cv = argmin([&](int c) { return ms[c][0] + ms[c][4]; });
-    const int cr = argmin([&](int c) { return ms[c][2]; });
-    const int cp = argmin([&](int c) { return ms[c][1] + ms[c][5]; });
-    const int cpr = argmin([&](int c) { return ms[c][3]; });
-    ss->bz_vel = cand[cv].first;
-    ss->bz_vel_recon = cand[cr].first;
-    ss->bz_pres = cand[cp].first;
-    ss->bz_pres_recon = cand[cpr].first;
-    ss->vec[0] = cand[cv].second;
-    ss->vec[1] = cand[cr].second;
-    ss->vec[2] = cand[cp].second;
-    ss->vec[3] = cand[cpr].second;
-    const std::array<int, 5> pick = {ss->bz_vel, ss->bz_vel_recon, ss->bz_pres, ss->bz_pres_recon, form_bits(ss)};
+    std::array<int, 4> best = {argmin([&](int c) { return ms[c][0] + ms[c][4]; }),
+                                     argmin([&](int c) { return ms[c][2]; }),
+                                     argmin([&](int c) { return ms[c][1] + ms[c][5]; }),
+                                     argmin([&](int c) { return ms[c][3]; })};
+    if (ss->vec[0] && ss->o.extra_images) {
+        // the wavefield decomposition decides on the signs of products near zero, and the forward
+        // pressure's interior tiles fuse one product (rtm_pipe.cu), so its tile height reaches the
+        // last bit of the fields: a fixed height by the batch's cells, 8 rows below 6 million (where
+        // 16 leave SMs idle) and 16 above
+        double cells = 0;
+        for (int j = 0; j < n; j++) cells += (double)ss->shots[k0 + j].X * ss->shots[k0 + j].Z;
+        best[2] = cells < 6e6 ? 8 : 16;
+    }
+    const auto use = [&](const std::array<int, 4> &h, bool merge) {
+        ss->bz_vel = h[0];
+        ss->bz_vel_recon = h[1];
+        ss->bz_pres = h[2];
+        ss->bz_pres_recon = h[3];
+        ss->merge = merge;
+    };
+    // whole steps of each plan
+    struct Plan {
+        std::array<int, 4> h;
+        bool merge;
+        float ms;
+    };
+    std::vector<Plan> plans = {{best, false, 0.f}};
+    if (ss->vec[0] && !ss->o.extra_images) {
+        plans.push_back({{8, 8, 8, 8}, true, 0.f});
+        plans.push_back({{16, 16, 16, 16}, true, 0.f});
+        cudaEvent_t e0, e1;
+        CK(cudaEventCreate(&e0));
+        CK(cudaEventCreate(&e1));
+        for (Plan &p : plans) {
+            use(p.h, p.merge);
+            BatchRun br;
+            if ((rc = batch_setup(ss, k0, n, br))) break;
+            StepArgs &a = br.a;
+            for (int it = -2; it < 6; it++) {
+                if (it == 0) cudaEventRecord(e0, st);
+                a.it = std::min(std::max(it, 0) + 1, ss->s.nt - 2);
+                a.tiles = ss->d_tiles;
+                vel_step(ss, RTM_WAVE_FWD, ss->bz_vel, a, br.ntiles);
+                a.tiles = ss->d_tiles_p;
+                pres_step(ss, RTM_WAVE_FWD, ss->bz_pres, a, br.ntiles_p, 0);
+                if (br.merged) {
+                    a.tiles = ss->d_tiles_m[0];
+                    pipe_step(ss, RTM_WAVE_RECON, RTM_WAVE_RECEIVER, ss->bz_vel, a, br.nmerged[0], 0);
+                    a.tiles = ss->d_tiles_m[1];
+                    pipe_step(ss, RTM_WAVE_RECEIVER, RTM_WAVE_RECON, ss->bz_vel, a, br.nmerged[1], 0);
+                } else {
+                    a.tiles = ss->d_tiles_r;
+                    vel_step(ss, RTM_WAVE_RECON, ss->bz_vel_recon, a, br.ntiles_r);
+                    a.tiles = ss->d_tiles_pr;
+                    pres_step(ss, RTM_WAVE_RECON, ss->bz_pres_recon, a, br.ntiles_pr, 0);
+                    a.tiles = ss->d_tiles;
+                    vel_step(ss, RTM_WAVE_RECEIVER, ss->bz_vel, a, br.ntiles);
+                    a.tiles = ss->d_tiles_p;
+                    pres_step(ss, RTM_WAVE_RECEIVER, ss->bz_pres, a, br.ntiles_p, 0);
+                }
+            }
+            cudaEventRecord(e1, st);
+            ss->launches += 8 * (br.merged ? 4 : 6);
+            if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+                rc = fail(RTM_ERR_CUDA, "tuner trial launches failed");
+                break;
+            }
+            cudaEventElapsedTime(&p.ms, e0, e1);
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (rc) return rc;
+        if ((rc = check_kernel_flag(ss))) return rc;
+    }
+    const Plan &plan = *std::min_element(plans.begin(), plans.end(), [](const Plan &x, const Plan &y) { return x.ms < y.ms; });
+    use(plan.h, plan.merge);
+    const std::array<int, 5> pick = {ss->bz_vel, ss->bz_vel_recon, ss->bz_pres, ss->bz_pres_recon,
+                                     form_bits(ss) | (ss->merge ? 16 : 0)};
     if (ss->o.verbose) {
-        std::printf("rtm_b200: tiles for %s: vel %d%s, vel_recon %d%s, pres %d%s, pres_recon %d%s (ms per 4 steps:",
-                    key.c_str(), pick[0], ss->vec[0] ? "v" : "s", pick[1], ss->vec[1] ? "v" : "s", pick[2],
-                    ss->vec[2] ? "v" : "s", pick[3], ss->vec[3] ? "v" : "s");
+        std::printf("rtm_b200: tiles for %s: vel %d, vel_recon %d, pres %d, pres_recon %d, %s launches (ms per 6 steps:",
+                    key.c_str(), pick[0], pick[1], pick[2], pick[3], ss->merge ? "merged" : "separate");
+        for (const Plan &p : plans) std::printf(" %s@%d/%d/%d/%d=%.3f", p.merge ? "merged" : "separate", p.h[0], p.h[1], p.h[2], p.h[3], p.ms);
+        std::printf("; ms per 4 steps:");
         for (int c = 0; c < nc; c++)
-            for (int k = 0; k < 6; k++)
-                std::printf(" %s@%d%s=%.3f", names[k], cand[c].first, cand[c].second ? "v" : "s", ms[c][k]);
+            for (int k = 0; k < 6; k++) std::printf(" %s@%dv=%.3f", names[k], cand[c], ms[c][k]);
         std::printf(")\n");
     }
     std::lock_guard<std::mutex> lock(g_tune_mu);

@@ -33,12 +33,16 @@ __device__ __forceinline__ float load_gather(const StepArgs &a, const ShotDev &S
 __global__ void k_setup_pml(float *pml, int X, int Z, int npml, float dx, float dz, float dt, float vpmax)
 {
     const PmlOffsets o = pml_offsets(X, Z);
-    const int n = X > Z ? X : Z;
+    const int PX = o.ic2x - o.c1x, PZ = o.ic2z - o.c1z, n = PX > PZ ? PX : PZ;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         for (int axis = 0; axis < 2; axis++) {
             const int L = axis == 0 ? X : Z;
             const float h = axis == 0 ? dx : dz;
-            if (i >= L) continue;
+            if (i >= L) {   // the padding
+                if (axis == 0 && i < PX) pml[o.c1x + i] = pml[o.ic2x + i] = pml[o.c1vx + i] = pml[o.ic2vx + i] = 1.0f;
+                if (axis == 1 && i < PZ) pml[o.c1z + i] = pml[o.ic2z + i] = pml[o.c1vz + i] = pml[o.ic2vz + i] = 1.0f;
+                continue;
+            }
             float R_ = 1.0e-10;
             float d = npml * h;
             float d0 = 1.5 * vpmax * logf(1 / R_) / d;

@@ -8,13 +8,23 @@
 // list built for that bz.
 void launch_vel(int mode, int bz, const StepArgs &a, int ntiles, cudaStream_t s);
 void launch_pres(int mode, int bz, const StepArgs &a, int ntiles, int record, cudaStream_t s);
-// The same launches with four columns by U rows per thread (rtm_stencil_v.cu): same tile
-// lists, staged boxes and results, 32 * bz / U threads per block.
-void launch_vel4(int mode, int bz, const StepArgs &a, int ntiles, cudaStream_t s);
+// The pipelined form (rtm_pipe.cu) of the tiles of pressure mode pm and velocity mode vm (-1: none
+// of that kind; both: a merged list whose velocity tiles carry RTM_TILE_VEL): same results.
+// One translation unit per tile height.
+void launch_pipe_8(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
+void launch_pipe_16(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
+void launch_pipe_32(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
+void launch_pipe_64(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
+inline void launch_pipe(int pm, int vm, int bz, const StepArgs &a, int ntiles, int record, cudaStream_t s)
+{
+    if (bz == 16) launch_pipe_16(pm, vm, a, ntiles, record, s);
+    else if (bz == 8) launch_pipe_8(pm, vm, a, ntiles, record, s);
+    else if (bz == 64) launch_pipe_64(pm, vm, a, ntiles, record, s);
+    else launch_pipe_32(pm, vm, a, ntiles, record, s);
+}
 // A whole pass in one persistent launch (rtm_stencil.cu, k_pass): dir 0 the source pass, 1 the
 // backward pass.  Only at the default tile heights (32, 16, 16); returns false otherwise.
 bool launch_pass(int dir, const PassArgs &p, int bz_vel, int bz_vel_recon, int bz_pres, cudaStream_t s);
-void launch_pres4(int mode, int bz, const StepArgs &a, int ntiles, int record, cudaStream_t s);
 // One whole time step (velocities and pressure) of one wavefield (rtm_step.cu): reads the
 // shots' a / b fields, writes an / bn; tz rows per tile (16 or 32), 256 threads per block;
 // `fast`: the tile list holds only interior tiles (the branch-free instance).

@@ -135,7 +135,7 @@ __device__ __forceinline__ void vel_tile(const StepArgs &a, const TileRef t, flo
     // unroll four row groups, so that the z window's shift becomes register renaming within
     // them (measured 1.5-2.5% faster; the pressure kernels and the smaller tiles were not
     // faster that way, or spilled)
-    if (t.interior) {
+    if (t.interior & 1) {
 #pragma unroll (MODE == 3 || BZ < 32 ? 1 : 4)
         for (int z = z0; z < z0 + BZ; z += U) {
             float nir[U], nov[U], now[U];
@@ -285,7 +285,7 @@ __device__ __forceinline__ void pres_tile(const StepArgs &a, int record, const T
         const int z1 = min(z0 + BZ, Z);
         prefetch_rows(kappa, 4, z0, z1, x0, pitch, 1);
         prefetch_rows(W.p, 4, z0, z1, x0, pitch, 2);
-        if (MODE != 3 && !t.interior) {
+        if (MODE != 3 && !(t.interior & 1)) {
             prefetch_rows(W.sx, 4, z0, z1, x0, pitch, 3);
             prefetch_rows(W.sz, 4, z0, z1, x0, pitch, 4);
         }
@@ -368,7 +368,7 @@ __device__ __forceinline__ void pres_tile(const StepArgs &a, int record, const T
 #pragma unroll
     for (int j = 0; j < QN; j++) q[j] = colz[j * BX];
 
-    if (t.interior) {
+    if (t.interior & 1) {
 #pragma unroll 1
         for (int z = z0; z < z0 + BZ; z += U) {
             float nkk[U], np0[U], nps[U];

@@ -106,6 +106,15 @@ __device__ __forceinline__ bool tile_wait(unsigned long long *bar, int *err, uns
         if (mbar_done(bar, parity)) break;
     return false;
 }
+// Programmatic dependent launch: let the next kernel's blocks be set up; wait until the kernel
+// before this one has finished and its writes are visible (to the tensor memory accelerator
+// too).
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+}
 // Fixed-grid launches: true for the blocks past the batch's tile list (see StepArgs::counts).
 __device__ __forceinline__ bool tile_beyond(const StepArgs &a) { return a.counts && (int)blockIdx.x >= a.counts[a.list]; }
 

@@ -15,6 +15,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <cuda_runtime.h>
+
 #define RTM_RADIUS 10
 #define RTM_BX 128       // stencil tile width: columns (= threads) per block
 // rows per unrolled group of the velocity kernels (forward and receiver passes; the
@@ -59,6 +61,8 @@ enum RtmPrecision { RTM_FP32 = 0, RTM_FP16 = 1, RTM_BF16 = 2 };
 //   c1x[X], ic2x[X]     pressure x part       c1vx[X], ic2vx[X]   vx
 //   c1z[Z], ic2z[Z]     pressure z part       c1vz[Z], ic2vz[Z]   vz
 // plus the raw profiles ddx[X], ddz[Z], ddxvx[X], ddzvz[Z] (reference kernel.cu:174-269).
+// The coefficient arrays are padded with ones to whole tiles (128 columns, 64 rows), so that the
+// pipelined kernels copy a tile's part of each as one 16-byte aligned block.
 struct PmlOffsets {
     int c1x, ic2x, c1vx, ic2vx, c1z, ic2z, c1vz, ic2vz, ddx, ddz, ddxvx, ddzvz, total;
 };
@@ -66,10 +70,11 @@ struct PmlOffsets {
 __host__ __device__ inline PmlOffsets pml_offsets(int X, int Z)
 {
     PmlOffsets o;
-    o.c1x = 0; o.ic2x = X; o.c1vx = 2 * X; o.ic2vx = 3 * X;
-    o.c1z = 4 * X; o.ic2z = 4 * X + Z; o.c1vz = 4 * X + 2 * Z; o.ic2vz = 4 * X + 3 * Z;
-    o.ddx = 4 * X + 4 * Z; o.ddz = 5 * X + 4 * Z; o.ddxvx = 5 * X + 5 * Z; o.ddzvz = 6 * X + 5 * Z;
-    o.total = 6 * X + 6 * Z;
+    const int PX = (X + RTM_BX - 1) / RTM_BX * RTM_BX, PZ = (Z + 63) / 64 * 64;
+    o.c1x = 0; o.ic2x = PX; o.c1vx = 2 * PX; o.ic2vx = 3 * PX;
+    o.c1z = 4 * PX; o.ic2z = 4 * PX + PZ; o.c1vz = 4 * PX + 2 * PZ; o.ic2vz = 4 * PX + 3 * PZ;
+    o.ddx = 4 * PX + 4 * PZ; o.ddz = o.ddx + X; o.ddxvx = o.ddz + Z; o.ddzvz = o.ddxvx + X;
+    o.total = o.ddzvz + Z;
     return o;
 }
 
@@ -136,11 +141,18 @@ enum RtmAccum { RTM_ACC_FP32 = 0, RTM_ACC_FP64 = 1, RTM_ACC_KAHAN = 2, RTM_ACC_F
 // (whole-step kernel, per wavefield (A, B) and buffer (0, 1): STEP_*: p in the box of rows
 // z0-19 .. z0+TZ+18, columns x0-24 .. x0+151; STEPVX_*: vx, rows z0 .. z0+TZ-1, columns
 // x0-12 .. x0+139; STEPVZ_*: vz, rows z0-10 .. z0+TZ+9, columns x0 .. x0+127)
+// (pipelined kernels: the tile's own rows and 128 columns of the per-cell operands: IR* 1/rho and
+// K* kappa of the forward and backward models, *_OWN, *_SX, *_SZ the fields, G1 and ILLUM the
+// accumulators, each in the tile height of its kernel family)
 enum RtmTmap { RTM_TMAP_A_P = 0, RTM_TMAP_A_VX, RTM_TMAP_A_VZ, RTM_TMAP_B_P, RTM_TMAP_B_VX, RTM_TMAP_B_VZ,
                RTM_TMAP_A_P_RECON, RTM_TMAP_STEP_A0, RTM_TMAP_STEP_A1, RTM_TMAP_STEP_B0, RTM_TMAP_STEP_B1,
                RTM_TMAP_STEPVX_A0, RTM_TMAP_STEPVX_A1, RTM_TMAP_STEPVX_B0, RTM_TMAP_STEPVX_B1,
                RTM_TMAP_STEPVZ_A0, RTM_TMAP_STEPVZ_A1, RTM_TMAP_STEPVZ_B0, RTM_TMAP_STEPVZ_B1,
-               RTM_TMAP_A_VX_RECON, RTM_TMAP_A_VZ_RECON, RTM_TMAP_COUNT };
+               RTM_TMAP_A_VX_RECON, RTM_TMAP_A_VZ_RECON,
+               RTM_TMAP_IRF, RTM_TMAP_IRB, RTM_TMAP_A_VX_OWN, RTM_TMAP_A_VZ_OWN, RTM_TMAP_B_VX_OWN, RTM_TMAP_B_VZ_OWN,
+               RTM_TMAP_IRB_RECON, RTM_TMAP_A_VX_OWN_RECON, RTM_TMAP_A_VZ_OWN_RECON, RTM_TMAP_KF, RTM_TMAP_KB,
+               RTM_TMAP_A_P_OWN, RTM_TMAP_B_P_OWN, RTM_TMAP_KB_RECON, RTM_TMAP_A_P_OWN_RECON,
+               RTM_TMAP_A_SX, RTM_TMAP_A_SZ, RTM_TMAP_B_SX, RTM_TMAP_B_SZ, RTM_TMAP_G1, RTM_TMAP_ILLUM, RTM_TMAP_COUNT };
 #define RTM_TMAP_BYTES 128
 
 // One block's work: the tile of `shot` whose top-left cell is (x0, z0).  x0 is a multiple of
@@ -149,8 +161,19 @@ struct TileRef {
     int shot;
     int x0, z0;
     int interior;   // 1: the tile lies in the interior and holds no source, receiver or strip
-                    // cell, so the kernels take their branch-free body (set by the host)
+                    // cell, so the kernels take their branch-free body (set by the host); and, for
+                    // the pipelined kernels, RTM_TILE_* bits of what the other tiles hold
 };
+// TileRef.interior beyond bit 0 (pipelined kernels): columns in the x bands or at the right edge;
+// columns of reduced order; source cells; receivers; pressure tiles with PML cells, and with image
+// cells; a velocity tile (merged lists)
+#define RTM_TILE_XBAND 2
+#define RTM_TILE_XEDGE 4
+#define RTM_TILE_SRC 8
+#define RTM_TILE_REC 16
+#define RTM_TILE_BAND 32
+#define RTM_TILE_IMG 64
+#define RTM_TILE_VEL 256
 
 // Kernel-wide constants of one launch.
 struct StepArgs {
@@ -159,6 +182,7 @@ struct StepArgs {
     const float *wavelet;   // [nt]
     const float *coef;      // [10][10] zero-padded Liu-Yang table
     float c10[10];          // full-order (half-order 10) coefficients, read from the constant bank
+    float2 c2[10];          // the same, each as a packed pair
     float dt, dtx, dtz;
     int it;                 // time index
     int strip_prec, gather_prec, accum_fp64;
@@ -169,6 +193,9 @@ struct StepArgs {
     // counts == nullptr: the grid is the tile count
     const int *counts;
     int list;
+    unsigned *queue;        // two tile counters of the pipelined kernels: a launch takes tiles from
+    int qsel;               // queue[qsel] and clears the other one for the launch after it
+    int save;               // 1: the pipelined source-pass kernels save their tiles' strip cells
     int prefetch;           // 1: the stencil kernels prefetch their tile's operand rows into L2
 };
 
