@@ -324,8 +324,8 @@ class Session:
         return g
 
     def images(self):
-        n = (self.survey.nz, self.survey.nx)
-        out = [np.zeros(n, np.float32) for _ in range(4)]
+        # one block for the four images: large allocations get huge pages
+        out = list(np.zeros((4, self.survey.nz, self.survey.nx), np.float32))
         _check(lib().rtm_session_get_images(self.h, *[_ptr(a) for a in out]))
         return dict(zip(("image1", "image2s", "image2m", "illum"), out))
 
@@ -339,8 +339,7 @@ class Session:
 
     def images_extra(self):
         """The other imaging conditions' stacked images (options.extra_images != 0)."""
-        n = (self.survey.nz, self.survey.nx)
-        out = [np.zeros(n, np.float32) for _ in self.EXTRA_IMAGES]
+        out = list(np.zeros((len(self.EXTRA_IMAGES), self.survey.nz, self.survey.nx), np.float32))
         _check(lib().rtm_session_get_images_extra(self.h, *[_ptr(a) for a in out]))
         return dict(zip(self.EXTRA_IMAGES, out))
 

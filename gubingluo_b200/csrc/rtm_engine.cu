@@ -2149,8 +2149,8 @@ int rtm_session_get_gather(rtm_session *ss, int k, float *gather)
     CK(cudaSetDevice(ss->dev));
     CK(cudaStreamSynchronize(ss->stream));
     const float *src = ss->s.mode == 0 ? sh.gather_raw : sh.gather32;
-    CK(cudaMemcpy(gather, src, sizeof(float) * (size_t)ss->s.nt * sh.g.nrec, cudaMemcpyDeviceToHost));
-    return RTM_OK;
+    const size_t n = sizeof(float) * (size_t)ss->s.nt * sh.g.nrec;
+    return copy_out(gather, src, n, n, 1);
 }
 
 int rtm_session_get_pml(rtm_session *ss, int k, float *ddx, float *ddz, float *ddxvx, float *ddzvz)
@@ -2190,15 +2190,8 @@ int rtm_session_nrec(rtm_session *ss, int k)
 static int copy_image(rtm_session *ss, void *dev, float *out)
 {
     if (!out) return RTM_OK;
-    size_t n = (size_t)ss->s.nx * ss->s.nz;
-    if (ss->o.accum_fp64) {
-        std::vector<double> t(n);
-        CK(cudaMemcpy(t.data(), dev, n * 8, cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < n; i++) out[i] = (float)t[i];
-    } else {
-        CK(cudaMemcpy(out, dev, n * 4, cudaMemcpyDeviceToHost));
-    }
-    return RTM_OK;
+    const size_t n = (size_t)ss->s.nx * ss->s.nz;
+    return copy_out(out, dev, 4 * n, 4 * n, 1, ss->o.accum_fp64 != 0);
 }
 
 int rtm_session_get_images(rtm_session *ss, float *image1, float *image2s, float *image2m, float *illum)
@@ -2221,9 +2214,11 @@ int rtm_session_get_images_f64(rtm_session *ss, double *image1, double *image2s,
     CK(cudaSetDevice(ss->dev));
     CK(cudaStreamSynchronize(ss->stream));
     size_t n = (size_t)ss->s.nx * ss->s.nz * 8;
-    if (image1) CK(cudaMemcpy(image1, ss->img1, n, cudaMemcpyDeviceToHost));
-    if (image2s) CK(cudaMemcpy(image2s, ss->img2s, n, cudaMemcpyDeviceToHost));
-    if (illum) CK(cudaMemcpy(illum, ss->illum, n, cudaMemcpyDeviceToHost));
+    double *out[3] = {image1, image2s, illum};
+    void *dev[3] = {ss->img1, ss->img2s, ss->illum};
+    for (int k = 0; k < 3; k++)
+        if (out[k])
+            if (int rc = copy_out(out[k], dev[k], n, n, 1)) return rc;
     return RTM_OK;
 }
 
@@ -2461,17 +2456,11 @@ int rtm_forward(const rtm_survey *s, const rtm_options *o, int ishot, const floa
         if (e != cudaSuccess) rc = fail(RTM_ERR_CUDA, cudaGetErrorString(e));
         if (!rc) rc = check_kernel_flag(ss);
         const size_t w = sizeof(float);
-        if (!rc && p && cudaMemcpy2D(p, sh.X * w, sl.a.p, sh.pitch * w, sh.X * w, sh.Z, cudaMemcpyDeviceToHost))
-            rc = fail(RTM_ERR_CUDA, "copy p");
-        if (!rc && vx &&
-            cudaMemcpy2D(vx, (sh.X - 1) * w, sl.a.vx, sh.pitch * w, (sh.X - 1) * w, sh.Z, cudaMemcpyDeviceToHost))
-            rc = fail(RTM_ERR_CUDA, "copy vx");
-        if (!rc && vz && cudaMemcpy2D(vz, sh.X * w, sl.a.vz, sh.pitch * w, sh.X * w, sh.Z - 1, cudaMemcpyDeviceToHost))
-            rc = fail(RTM_ERR_CUDA, "copy vz");
-        if (!rc && gather &&
-            cudaMemcpy(gather, s->mode == 0 ? sh.gather_raw : sh.gather32, w * (size_t)nsteps * sh.g.nrec,
-                       cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = fail(RTM_ERR_CUDA, "copy gather");
+        if (!rc && p) rc = copy_out(p, sl.a.p, sh.pitch * w, sh.X * w, sh.Z);
+        if (!rc && vx) rc = copy_out(vx, sl.a.vx, sh.pitch * w, (sh.X - 1) * w, sh.Z);
+        if (!rc && vz) rc = copy_out(vz, sl.a.vz, sh.pitch * w, sh.X * w, sh.Z - 1);
+        const size_t g = w * (size_t)nsteps * sh.g.nrec;
+        if (!rc && gather) rc = copy_out(gather, s->mode == 0 ? sh.gather_raw : sh.gather32, g, g, 1);
     }
     rtm_session_close(ss);
     return rc;

@@ -1,5 +1,6 @@
 // rtm_internal.h — declarations shared by the library's translation units.
 #pragma once
+#include <cstddef>
 #include <string>
 #include <utility>
 #include <vector>
@@ -24,6 +25,9 @@ void interp_model(const float *vp0, float *vp, int nx0, int nz0, int nx, int lx,
 void get_constant(const float *vp, float fdom, float dx0, float dz0, int nx0, int nz0, int nt0, float dt0,
                   float *dx, float *dz, int *nx, int *nz, int *nt, float *dt, int *lx, int *lz, float *vpmin,
                   float *vpmax);
+// Device rows into packed host rows (rtm_copy.cu); narrow: doubles into floats.
+int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, size_t rows, bool narrow = false);
+
 void laplace_image(float *image, int nx, int nz, int dx, int dz);
 void scale_image(const float *illum, float *grad, int n);
 

@@ -425,11 +425,14 @@ extern "C" int rtm_interp_gather(const float *seisobs, int nx0, int nt0, float *
     if (cudaMalloc(&d_out, sizeof(float) * (size_t)nt * nx) != cudaSuccess)
         rc = fail(RTM_ERR_NOMEM, "rtm_interp_gather: device allocation failed");
     if (!rc) rc = interp_gather_device(p, seisobs, nx0, nt0, d_out, nx, nt, dt, dt0, mirror, st, nullptr);
-    if (!rc && cudaStreamSynchronize(st) == cudaSuccess) rc = interp_check_guards(p);
     if (!rc) {
-        cudaError_t e = cudaMemcpyAsync(seiscal, d_out, sizeof(float) * (size_t)nt * nx, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) rc = fail(RTM_ERR_CUDA, std::string("rtm_interp_gather: ") + cudaGetErrorString(e));
+        cudaError_t e = cudaStreamSynchronize(st);
+        rc = e == cudaSuccess ? interp_check_guards(p)
+                              : fail(RTM_ERR_CUDA, std::string("rtm_interp_gather: ") + cudaGetErrorString(e));
+    }
+    if (!rc) {
+        const size_t n = sizeof(float) * (size_t)nt * nx;
+        rc = copy_out(seiscal, d_out, n, n, 1);
     }
     p.release();
     if (d_out) cudaFree(d_out);
