@@ -52,13 +52,15 @@ struct InterpShape {
 };
 int interp_shape(int nx0, int nt0, int nx, int nt, InterpShape &sh);
 
-// Device workspace and cuFFT plans of one shape; kept by the caller and reused while the
+// Device workspace (and cuFFT plans beyond rtm_fk.cuh's lengths) of one shape; kept by the caller and reused while the
 // shape repeats (shots of a survey usually share it).
 struct InterpPlan {
     InterpShape shape{};
     void *work = nullptr;                 // one allocation holding everything below
-    float *d_in = nullptr, *d_tmp = nullptr;
+    float *d_in = nullptr, *d_tmp = nullptr, *d_out = nullptr;
     void *K = nullptr, *S = nullptr, *Z = nullptr, *G1 = nullptr, *G = nullptr;   // double2 arrays
+    void *A = nullptr, *tw = nullptr, *chirp[3] = {nullptr, nullptr, nullptr};   // rtm_fk.cuh's tables
+    int mt = 0;
     unsigned *zmax = nullptr;
     int p_k = 0, p_s = 0, p_x = 0, p_t = 0;   // cufftHandle values, valid when `plans`
     bool plans = false;
@@ -67,8 +69,8 @@ struct InterpPlan {
 };
 // Checking mode (RTM_B200_GUARDS=1): the guard bands after the workspace's buffers are intact.
 int interp_check_guards(const InterpPlan &p);
-// Uploads host_in [nt0][nx0] and writes the interpolated gather to d_out [nt][nx] on stream
-// st; mirror 0 = the reference's negative-frequency indexing, 1 = the Hermitian partner.
+// Uploads host_in [nt0][nx0] and writes the interpolated gather to d_out [nt][nx] (nullptr: to
+// p.d_out, part of the workspace) on stream st; mirror 0 = the reference's negative-frequency indexing, 1 = the Hermitian partner.
 int interp_gather_device(InterpPlan &p, const float *host_in, int nx0, int nt0, float *d_out, int nx, int nt,
                          float dt, float dt0, int mirror, cudaStream_t_fwd st, int *launches);
 

@@ -2,8 +2,9 @@
 // (reference Interpseis2d / GeneralFKinterp / Sincinterp, Interp_function.cpp:10-264, which
 // run on the host with FFTW).  Used by the real-data path before the direct-wave mute.
 //
-//   x: general F-K interpolation by lx = (nx-1)/(nx0-1): cuFFT double-complex transforms
-//      (the reference's FFTW plans are double precision) around four kernels;
+//   x: general F-K interpolation by lx = (nx-1)/(nx0-1) in double precision (the reference's
+//      FFTW plans are): the transforms of rtm_fk.cuh up to its longest length, beyond it cuFFT
+//      around four kernels;
 //   t: 21-tap Kaiser-windowed sinc, one thread per output sample.
 //
 // Expressions follow the reference's float/double evaluation; products and sums that the
@@ -19,11 +20,15 @@
 #include <string>
 
 #include "rtm_b200.h"
+#include "rtm_fk.cuh"
 #include "rtm_internal.h"
 
 namespace rtm {
 
 namespace {
+
+// The transforms of rtm_fk.cuh reach the shape's lengths (the padded width is the longer one in x).
+bool own_transforms(const InterpShape &sh) { return sh.nt0 <= fk::kMaxN && sh.Nx <= fk::kMaxN; }
 
 constexpr int kTaps = 21;
 struct Kaiser21 {
@@ -125,11 +130,7 @@ __global__ void k_fk_load(const float *__restrict__ in, double2 *__restrict__ K,
     S[i] = make_double2(v, 0.0);
 }
 
-// |z| as the reference's fftw_fabs: sqrtf of the float-rounded double re^2 + im^2.
-__device__ __forceinline__ float cabs_f(double re, double im)
-{
-    return sqrtf(__double2float_rn(__dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im))));
-}
+using fk::cabs_f;
 
 // F-K step 2a: Z [nx0][Nt] = (sum of the lx aliased rows of S) / lx, and max |Z| (the lx
 // copies of Z that the reference keeps are identical).  Non-negative floats order like
@@ -274,10 +275,12 @@ int interp_shape(int nx0, int nt0, int nx, int nt, InterpShape &sh)
     return RTM_OK;
 }
 
-// Device workspace and cuFFT plans for one interpolation shape (kept while the shape repeats).
-static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st)
+// Device workspace and cuFFT plans for one interpolation shape (kept while the shape repeats);
+// with_out: room for the result too (p.d_out).
+static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool with_out)
 {
-    if (p.work && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (!sh.fk || p.plans)) {
+    const bool own = sh.fk && own_transforms(sh);
+    if (p.work && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (!sh.fk || own || p.plans)) {
         if (p.plans) {
             CKF(cufftSetStream((cufftHandle)p.p_k, st));
             CKF(cufftSetStream((cufftHandle)p.p_s, st));
@@ -301,8 +304,24 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st)
         return o;
     };
     const size_t o_in = take(sizeof(float) * (size_t)sh.nt0 * sh.nx0);
+    const size_t o_out = with_out ? take(sizeof(float) * (size_t)sh.nt * sh.nx) : 0;
     size_t o_tmp = 0, o_K = 0, o_S = 0, o_Z = 0, o_G1 = 0, o_G = 0, o_zm = 0;
-    if (sh.fk) {
+    size_t o_A = 0, o_tw = 0, o_c[3] = {0, 0, 0};
+    const int len[3] = {sh.nt0, sh.nx0, sh.Nx};
+    int mt = 16;
+    if (own) {
+        const size_t nh = sh.Nt / 2 + 1;
+        for (int l : len) mt = std::max(mt, fk::pow2_for(l));
+        o_tmp = take(sizeof(float) * (size_t)sh.nt0 * sh.nx);
+        o_A = take(sizeof(double2) * nh * sh.nx0);
+        o_K = take(sizeof(double2) * (size_t)sh.nf * sh.nx0);
+        o_S = take(sizeof(double2) * (size_t)sh.nf * sh.Nx);
+        o_Z = take(sizeof(double2) * (size_t)sh.nf * sh.nx0);
+        o_G = take(sizeof(double2) * (size_t)sh.nf * sh.nx);
+        o_tw = take(sizeof(double2) * (mt / 4));
+        for (int k = 0; k < 3; k++) o_c[k] = take(sizeof(double2) * fk::pow2_for(len[k]));
+        o_zm = take(sizeof(unsigned));
+    } else if (sh.fk) {
         o_tmp = take(sizeof(float) * (size_t)sh.nt0 * sh.nx);
         o_K = take(sizeof(double2) * (size_t)sh.nx0 * sh.nt0);
         o_S = take(sizeof(double2) * (size_t)sh.Nx * sh.Nt);
@@ -315,7 +334,32 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st)
     char *b = (char *)p.work;
     for (const auto &g : p.guards) CKI(cudaMemsetAsync(b + g.first, 0xA5, g.second, st));
     p.d_in = (float *)(b + o_in);
-    if (sh.fk) {
+    p.d_out = with_out ? (float *)(b + o_out) : nullptr;
+    if (own) {
+        p.d_tmp = (float *)(b + o_tmp);
+        p.A = b + o_A;
+        p.K = b + o_K;
+        p.S = b + o_S;
+        p.Z = b + o_Z;
+        p.G = b + o_G;
+        p.tw = b + o_tw;
+        p.zmax = (unsigned *)(b + o_zm);
+        p.mt = mt;
+        fk::ChirpArgs ca;
+        for (int k = 0; k < 3; k++) {
+            p.chirp[k] = b + o_c[k];
+            ca.len[k] = len[k];
+            ca.out[k] = (double2 *)p.chirp[k];
+        }
+        const size_t smem = fk::smem_bytes(mt);
+        // (attributes of the instances on this device; setting them again is harmless)
+        CKI(cudaFuncSetAttribute(fk::k_chirps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        for (auto *f : {fk::k_fk_time, fk::k_fk_space, fk::k_fk_filter, fk::k_fk_back})
+            CKI(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        fk::k_twiddles<<<8, 256, 0, st>>>((double2 *)p.tw, mt);
+        fk::k_chirps<<<3, 512, smem, st>>>(ca, (const double2 *)p.tw, mt);
+        CKI(cudaGetLastError());
+    } else if (sh.fk) {
         p.d_tmp = (float *)(b + o_tmp);
         p.K = b + o_K;
         p.S = b + o_S;
@@ -360,7 +404,32 @@ static int interp_run(InterpPlan &p, float *out, float dt, float dt0, int mirror
     const int T = 256;
     const float *src = p.d_in;
     int ld = sh.nx0;
-    if (sh.fk) {
+    if (sh.fk && own_transforms(sh)) {
+        const int rows = sh.sinc ? sh.nt0 : std::min(sh.nt, sh.nt0);
+        fk::FkArgs a{};
+        a.in = p.d_in;
+        a.nx0 = sh.nx0; a.nt0 = sh.nt0; a.nx = sh.nx; a.lx = sh.lx; a.Nx = sh.Nx; a.Nt = sh.Nt; a.nf = sh.nf;
+        a.nh = sh.Nt / 2 + 1;
+        a.rows = rows;
+        a.mirror = mirror;
+        a.A = (double2 *)p.A; a.K = (double2 *)p.K; a.S = (double2 *)p.S; a.Z = (double2 *)p.Z; a.G = (double2 *)p.G;
+        a.zmax = p.zmax;
+        a.ct = (const double2 *)p.chirp[0]; a.cx = (const double2 *)p.chirp[1]; a.cX = (const double2 *)p.chirp[2];
+        a.tw = (const double2 *)p.tw;
+        a.mt = p.mt;
+        a.out = sh.sinc ? p.d_tmp : out;
+        CKI(cudaMemsetAsync(p.zmax, 0, sizeof(unsigned), st));
+        const int mT = fk::pow2_for(sh.nt0), mx = fk::pow2_for(sh.nx0), mX = fk::pow2_for(sh.Nx);
+        // threads: one radix-4 butterfly each per stage up to 512 (warps are whole)
+        const auto threads = [](int m) { return std::min(512, std::max(32, m / 4)); };
+        fk::k_fk_time<<<dim3(sh.nx0, sh.lx), threads(mT), fk::smem_bytes(mT), st>>>(a);
+        fk::k_fk_space<<<a.nh, threads(mx), fk::smem_bytes(mx), st>>>(a);
+        fk::k_fk_filter<<<sh.nf, threads(mX), fk::smem_bytes(mX), st>>>(a);
+        fk::k_fk_back<<<sh.nx, threads(mT), fk::smem_bytes(mT), st>>>(a);
+        if (launches) *launches += 4;
+        src = p.d_tmp;
+        ld = sh.nx;
+    } else if (sh.fk) {
         double2 *K = (double2 *)p.K, *S = (double2 *)p.S, *Z = (double2 *)p.Z, *G1 = (double2 *)p.G1,
                 *G = (double2 *)p.G;
         CKI(cudaMemsetAsync(p.zmax, 0, sizeof(unsigned), st));
@@ -398,8 +467,9 @@ int interp_gather_device(InterpPlan &p, const float *host_in, int nx0, int nt0, 
     InterpShape sh;
     int rc = interp_shape(nx0, nt0, nx, nt, sh);
     if (rc) return rc;
-    rc = plan_for(p, sh, st);
+    rc = plan_for(p, sh, st, !d_out);
     if (rc) return rc;
+    if (!d_out) d_out = p.d_out;
     CKI(cudaMemcpyAsync(p.d_in, host_in, sizeof(float) * (size_t)nt0 * nx0, cudaMemcpyHostToDevice, st));
     return interp_run(p, d_out, dt, dt0, mirror, st, launches);
 }
@@ -420,11 +490,7 @@ extern "C" int rtm_interp_gather(const float *seisobs, int nx0, int nt0, float *
     cudaStream_t st;
     CKI(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     InterpPlan p;
-    float *d_out = nullptr;
-    int rc = RTM_OK;
-    if (cudaMalloc(&d_out, sizeof(float) * (size_t)nt * nx) != cudaSuccess)
-        rc = fail(RTM_ERR_NOMEM, "rtm_interp_gather: device allocation failed");
-    if (!rc) rc = interp_gather_device(p, seisobs, nx0, nt0, d_out, nx, nt, dt, dt0, mirror, st, nullptr);
+    int rc = interp_gather_device(p, seisobs, nx0, nt0, nullptr, nx, nt, dt, dt0, mirror, st, nullptr);
     if (!rc) {
         cudaError_t e = cudaStreamSynchronize(st);
         rc = e == cudaSuccess ? interp_check_guards(p)
@@ -432,10 +498,9 @@ extern "C" int rtm_interp_gather(const float *seisobs, int nx0, int nt0, float *
     }
     if (!rc) {
         const size_t n = sizeof(float) * (size_t)nt * nx;
-        rc = copy_out(seiscal, d_out, n, n, 1);
+        if (!rc) rc = copy_out(seiscal, p.d_out, n, n, 1);
     }
     p.release();
-    if (d_out) cudaFree(d_out);
     cudaStreamDestroy(st);
     return rc;
 }
