@@ -1563,8 +1563,10 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
             ss->launches += 3;
             flush_images(it);
             if (o.extra_images) {
+                timing_begin(ss, "image_extra", it, &e);
                 launch_image_extra(ss->d_shots, n, br.ex_nxi, br.ex_nzi, o.extra_images == 2, o.accum_fp64, s.dx, s.dz,
                                    s.dt, st);
+                timing_end(ss, e);
                 ss->launches++;
             }
         }

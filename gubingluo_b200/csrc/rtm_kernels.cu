@@ -360,7 +360,7 @@ __global__ void k_finalize_extra(const FinalizeShot *fs, int nshots, int nx, int
 
 // The reference's other imaging conditions for one backward step (kernel.cu:1417-1522;
 // rtm_model.cu:450-455), run after the receiver update on the interior of every shot of a
-// batch, one thread per cell, grid (ceil(nxi/32), ceil(nzi/8), nshots):
+// batch, grid (ceil((nxi + 3) / 128), ceil(nzi/8), nshots):
 //   g2  += the up-down, down-up, left-right and right-left products of the decomposed
 //          pressures (the reference keeps four arrays and adds them at the end);
 //   g3  += ps p cos(theta), theta from the angle between the source and receiver Poynting
@@ -373,61 +373,150 @@ __global__ void k_finalize_extra(const FinalizeShot *fs, int nshots, int nx, int
 // vx and vz at the cell itself.  Operand types follow the reference's expressions (float
 // values, double literals).  Each cell's pressures then become the "before" values of the
 // next (earlier) step.
+//
+// A thread takes four adjacent columns (16-byte words; the neighbours in x from its own words and
+// two single loads), a warp 128 columns of a row.  A quotient of two floats that the reference
+// forms in double and rounds to float is the correctly rounded float quotient (double has more
+// than twice a float's digits), so those divisions are float ones; what stays in double is the
+// angle's complement, the true-amplitude term and the quotient by the double 1e-6.  Zeros, which
+// fill most of both wavefields for much of the pass and which the library's division and root
+// take through their slow branches, are answered directly.  Measured with one cell per thread and
+// all of it in double: 78 us per step for 8 shots of 801 x 301 at 700 instructions per cell; now 47 us
+// at 230 (76 bytes per cell: 23 us at the memory's rate), bound by instructions and by the
+// latency of their branches at 16 warps per SM.
+__device__ __forceinline__ void ld_row4(const float *f, size_t id, float (&v)[4])
+{
+    const float4 t = *(const float4 *)(f + id);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void ld_row4(const double *f, size_t id, double (&v)[4])
+{
+    const double2 t = *(const double2 *)(f + id), u = *(const double2 *)(f + id + 2);
+    v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
+}
+__device__ __forceinline__ void st_row4(float *f, size_t id, const float (&v)[4])
+{
+    *(float4 *)(f + id) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void st_row4(double *f, size_t id, const double (&v)[4])
+{
+    *(double2 *)(f + id) = make_double2(v[0], v[1]);
+    *(double2 *)(f + id + 2) = make_double2(v[2], v[3]);
+}
+
+// RN(a / b) for b > 0 given rb = RN(1 / b): two of Markstein's correction steps (exact residual by a
+// fused multiply-add; a faithful quotient so corrected is the rounded one), in the range where no
+// residual underflows; zero, which sends the library's division down its slow branch, is itself.
+__device__ __forceinline__ float div_by(float a, float b, float rb)
+{
+    if (fabsf(a) >= 1.0e-25f && fabsf(a) < 1.0e25f) {
+        float q = __fmul_rn(a, rb);
+        q = __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
+        return __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
+    }
+    return a == 0.0f ? a : __fdiv_rn(a, b);
+}
+
 template <int PAR, typename ACC>
-__global__ void k_image_extra(const ShotDev *shots, float dx, float dz, float dt)
+__global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float dx, float dz, float dt)
 {
     const ShotDev &S = shots[blockIdx.z];
-    const int ix = blockIdx.x * 32 + threadIdx.x, iz = blockIdx.y * 8 + threadIdx.y;
-    if (ix >= S.nxi || iz >= S.nzi) return;
     const int X = S.X, pitch = S.pitch, npml = S.npml;
-    const int z = iz + npml, x = ix + npml;
-    const size_t id = (size_t)z * pitch + x;
-    size_t ivx = id;
+    const int x0 = (npml & ~3) + 4 * (int)(blockIdx.x * 32 + threadIdx.x), iz = blockIdx.y * 8 + threadIdx.y;
+    if (x0 >= X - npml || iz >= S.nzi) return;   // (x0 + 3 lies inside the row pitch)
+    const int z = iz + npml;
+    const size_t id = (size_t)z * pitch + x0;
+    const float *ap = S.a.p, *bp = S.b.p;
+    float ps[4], p[4], vxs[4], vx[4], vzs[4], vz[4], v2[4], pspre[4], ppre[4];
+    float psu4[4], psd4[4], pu4[4], pd4[4];   // the rows above and below
+    ld_row4(ap, id, ps);
+    ld_row4(bp, id, p);
+    ld_row4(S.a.vz, id, vzs);
+    ld_row4(S.b.vz, id, vz);
+    ld_row4(S.vp2_b, id, v2);
+    ld_row4(S.ps_pre, id, pspre);
+    ld_row4(S.p_pre, id, ppre);
+    ld_row4(ap, id - pitch, psu4);
+    ld_row4(ap, id + pitch, psd4);
+    ld_row4(bp, id - pitch, pu4);
+    ld_row4(bp, id + pitch, pd4);
+    const float psl = ap[id - 1], psr = ap[id + 4], pl_ = bp[id - 1], pr_ = bp[id + 4];
     if (PAR) {
-        const long f = (long)z * X + x;
-        ivx = (size_t)(f / (X - 1)) * pitch + (size_t)(f % (X - 1));
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const long f = (long)z * X + min(x0 + j, X - npml - 1);
+            const size_t ivx = (size_t)(f / (X - 1)) * pitch + (size_t)(f % (X - 1));
+            vxs[j] = S.a.vx[ivx];
+            vx[j] = S.b.vx[ivx];
+        }
+    } else {
+        ld_row4(S.a.vx, id, vxs);
+        ld_row4(S.b.vx, id, vx);
     }
-    const float ps = S.a.p[id], p = S.b.p[id];
-    const float vxs = S.a.vx[ivx], vx = S.b.vx[ivx], vzs = S.a.vz[id], vz = S.b.vz[id];
-    const float v2 = S.vp2_b[id];
-    ACC *g2 = (ACC *)S.gx[0], *g3 = (ACC *)S.gx[1], *g3t = (ACC *)S.gx[2], *g4 = (ACC *)S.gx[3];
-    // decomposition (kernel.cu:1417-1451)
-    {
-        const float vectxs = -ps * vxs, vectzs = -ps * vzs, vectxr = -p * vx, vectzr = -p * vz;
-        const float psu = vectzs < 0 ? ps : 0.0f, psd = vectzs > 0 ? ps : 0.0f;
-        const float psl = vectxs < 0 ? ps : 0.0f, psr = vectxs > 0 ? ps : 0.0f;
-        const float pu = vectzr < 0 ? p : 0.0f, pd = vectzr > 0 ? p : 0.0f;
-        const float pl = vectxr < 0 ? p : 0.0f, pr = vectxr > 0 ? p : 0.0f;
-        g2[id] += (ACC)(psu * pd + psd * pu + psl * pr + psr * pl);
-    }
-    // Poynting angle (kernel.cu:1452-1485)
-    {
-        const float ksx = ps * vxs, ksz = ps * (PAR ? vz : vzs), krx = p * vx, krz = p * vz;
-        const float q = (ksx * ksx + ksz * ksz) * (krx * krx + krz * krz);
-        const double den = sqrtf(q) > 0 ? (double)sqrtf(q) : 1.0e-6;
-        float wt = (float)((double)(ksx * krx + ksz * krz) / den);
-        if (wt >= -1.0 && wt <= 1.0) {
-            wt = (float)(0.5 * (double)acosf(wt));
-            wt = (float)(RTM_PI / 2.0 - (double)wt);
-            if (wt > 0 && wt <= RTM_PI / 3.0) {
-                const float c = ps * p * cosf(wt);
-                const double t = (double)(ps * p) * 16.0 * RTM_PI * (double)sqrtf(v2) / (double)sinf(wt);
-                g3[id] += (ACC)c;
-                g3t[id] = (ACC)((double)g3t[id] + t);
+    const float w0 = (float)(RTM_PI / 2.0 - (double)(0.5f * acosf(0.0f))), c0 = cosf(w0), s0 = sinf(w0);
+    const float rdx = __frcp_rn(dx), rdz = __frcp_rn(dz);
+    ACC *g2p = (ACC *)S.gx[0], *g3p = (ACC *)S.gx[1], *g3tp = (ACC *)S.gx[2], *g4p = (ACC *)S.gx[3];
+    ACC g2[4], g3[4], g3t[4], g4[4];
+    ld_row4(g2p, id, g2);
+    ld_row4(g3p, id, g3);
+    ld_row4(g3tp, id, g3t);
+    ld_row4(g4p, id, g4);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (x0 + j < npml || x0 + j >= X - npml) continue;
+        // decomposition (kernel.cu:1417-1451)
+        {
+            const float vectxs = -ps[j] * vxs[j], vectzs = -ps[j] * vzs[j], vectxr = -p[j] * vx[j], vectzr = -p[j] * vz[j];
+            const float psu = vectzs < 0 ? ps[j] : 0.0f, psd = vectzs > 0 ? ps[j] : 0.0f;
+            const float psl = vectxs < 0 ? ps[j] : 0.0f, psr = vectxs > 0 ? ps[j] : 0.0f;
+            const float pu = vectzr < 0 ? p[j] : 0.0f, pd = vectzr > 0 ? p[j] : 0.0f;
+            const float pl = vectxr < 0 ? p[j] : 0.0f, pr = vectxr > 0 ? p[j] : 0.0f;
+            g2[j] += (ACC)(psu * pd + psd * pu + psl * pr + psr * pl);
+        }
+        // Poynting angle (kernel.cu:1452-1485)
+        {
+            const float ksx = ps[j] * vxs[j], ksz = ps[j] * (PAR ? vz[j] : vzs[j]), krx = p[j] * vx[j], krz = p[j] * vz[j];
+            const float q = (ksx * ksx + ksz * ksz) * (krx * krx + krz * krz);
+            const float num = ksx * krx + ksz * krz;
+            // where the product under the root underflows, num / 1e-6 is tiny, and acosf of anything
+            // below 1e-8 is acosf(0) (compared for every float): one angle, w0, for all those cells
+            // (the root of zero, which takes the slow branch of sqrtf, is not formed)
+            const bool under = !(q > 0), tiny = under && fabsf(num) < 7.0e-15f;
+            float wt = w0;
+            bool in = true;
+            if (!tiny) {
+                wt = under ? (float)((double)num / 1.0e-6) : __fdiv_rn(num, sqrtf(q));
+                in = wt >= -1.0f && wt <= 1.0f;
+                if (in) {
+                    wt = 0.5f * acosf(wt);
+                    wt = (float)(RTM_PI / 2.0 - (double)wt);
+                    in = wt > 0 && wt <= RTM_PI / 3.0;
+                }
+            }
+            const float pp = ps[j] * p[j];
+            if (in && pp != 0.0f) {   // (a zero product adds nothing)
+                const float cw = tiny ? c0 : cosf(wt), sw = tiny ? s0 : sinf(wt);
+                g3[j] += (ACC)(pp * cw);
+                g3t[j] = (ACC)((double)g3t[j] + (double)pp * 16.0 * RTM_PI * (double)sqrtf(v2[j]) / (double)sw);
             }
         }
+        // energy norm (kernel.cu:1486-1522)
+        {
+            const float psx = div_by(0.5f * ((j < 3 ? ps[j + 1] : psr) - (j > 0 ? ps[j - 1] : psl)), dx, rdx);
+            const float psz = div_by(0.5f * (psd4[j] - psu4[j]), dz, rdz);
+            const float px = div_by(0.5f * ((j < 3 ? p[j + 1] : pr_) - (j > 0 ? p[j - 1] : pl_)), dx, rdx);
+            const float pz = div_by(0.5f * (pd4[j] - pu4[j]), dz, rdz);
+            const float dd = -(ps[j] - pspre[j]) * (p[j] - ppre[j]);
+            const float e = dd == 0.0f ? dd : dd / (dt * dt * v2[j]);
+            g4[j] += (ACC)(e + psx * px + psz * pz);
+        }
     }
-    // energy norm (kernel.cu:1486-1522)
-    {
-        const float *ap = S.a.p, *bp = S.b.p;
-        const float psx = (float)(0.5 * (double)(ap[id + 1] - ap[id - 1]) / dx);
-        const float psz = (float)(0.5 * (double)(ap[id + pitch] - ap[id - pitch]) / dz);
-        const float px = (float)(0.5 * (double)(bp[id + 1] - bp[id - 1]) / dx);
-        const float pz = (float)(0.5 * (double)(bp[id + pitch] - bp[id - pitch]) / dz);
-        g4[id] += (ACC)(-(ps - S.ps_pre[id]) * (p - S.p_pre[id]) / (dt * dt * v2) + psx * px + psz * pz);
-    }
-    S.ps_pre[id] = ps;
-    S.p_pre[id] = p;
+    st_row4(g2p, id, g2);
+    st_row4(g3p, id, g3);
+    st_row4(g3tp, id, g3t);
+    st_row4(g4p, id, g4);
+    st_row4(S.ps_pre, id, ps);
+    st_row4(S.p_pre, id, p);
 }
 
 // =====================================================================================
@@ -525,7 +614,8 @@ void launch_image_flush(const ShotDev *shots, int nshots, int max_nxi, int max_n
 void launch_image_extra(const ShotDev *shots, int nshots, int max_nxi, int max_nzi, int parity, int fp64,
                         float dx, float dz, float dt, cudaStream_t s)
 {
-    dim3 grid((max_nxi + 31) / 32, (max_nzi + 7) / 8, nshots), block(32, 8);
+    // (up to three columns before the interior's first belong to its first word)
+    dim3 grid((max_nxi + 3 + 127) / 128, (max_nzi + 7) / 8, nshots), block(32, 8);
     if (parity) {
         if (fp64) k_image_extra<1, double><<<grid, block, 0, s>>>(shots, dx, dz, dt);
         else k_image_extra<1, float><<<grid, block, 0, s>>>(shots, dx, dz, dt);

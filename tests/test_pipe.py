@@ -109,3 +109,23 @@ def test_images_and_fields_to_the_host(rtmlib, nx, nz, accum):
     with G.Session(s, G.RunOptions(), [1], v, rho) as ss:   # the same field through another copy
         ss.model()
         assert np.array_equal(ss.wavefields(0, nx + 20, nz + 20)[0], p)
+
+
+# the other imaging conditions take words of four columns: interiors that start and end at every
+# alignment, one word and partial last words, against the oracle
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,npml", [(61, 20), (62, 21), (63, 22), (64, 23), (125, 12), (129, 13), (3, 10)])
+@pytest.mark.parametrize("accum", [0, 1])
+def test_other_imaging_conditions_at_word_edges(rtmlib, oracle, nx, npml, accum):
+    G = rtmlib
+    nz = 41
+    v, rho = _models(nz, nx, nx)
+    s = _survey(G, nx, nz, npml, 130, spx0=(nx // 2) * 10.0, amp=1.0e4)
+    got = G.migrate(s, G.RunOptions(extra_images=1, accum_fp64=accum), [1], v, rho)
+    d = {k: getattr(s, k) for k in s.__dataclass_fields__}
+    want = oracle.rtm_model(d, [1], v, rho, extra=1)
+    # the tolerances of test_gpu_parity: 1e-4 where the terms are sums of products, 3e-3 where they
+    # switch on signs of rounded products
+    for k, tol in (("image1", 1e-4), ("image5s", 1e-4), ("image5m", 1e-4), ("image3m", 3e-3)):
+        a, b = got[k].astype(np.float64), want[k].astype(np.float64)
+        assert np.linalg.norm(b) > 0 and np.linalg.norm(a - b) <= tol * np.linalg.norm(b), k
