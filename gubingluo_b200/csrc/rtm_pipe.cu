@@ -25,7 +25,9 @@
 //     receiver velocity} and {receiver pressure with imaging, next step's reconstruction
 //     velocity}.
 //   * Launches use programmatic dependent launch: a kernel's blocks are set up while the kernel
-//     before it drains, and wait for its completion before they read any field.
+//     before it drains, and wait for its completion before they read any field; the first tile's
+//     copies of what no kernel of the pass writes (1/rho or kappa, damping factors) start before
+//     that wait.
 //
 // Reference kernels these replace: see rtm_stencil.cu.
 #include <atomic>
@@ -155,7 +157,7 @@ struct Stage {
 // Tiles of up to 16 rows stage what only some pressure tiles need as well: the split PML fields
 // of band tiles; ps, g1 and illum of the receiver pass's tiles with interior cells (which then
 // load their split fields, if any, directly, one row ahead).  Taller tiles have no room for it.
-template <int BZ, int PM, int VM, typename ACC>
+template <int BZ, int PM, int VM, typename ACC, bool THIN = false>
 struct Pipe {
     static constexpr bool staged = BZ <= 16;
     static constexpr int row = BZ * BX * 4;   // bytes of one operand of a tile
@@ -164,12 +166,12 @@ struct Pipe {
     // blocks of n stages that fit an SM's shared memory (a block's own part: descriptors, barriers,
     // coefficients and the system's 1 KB)
     static constexpr int fit(int n) { return 228 * 1024 / (n * bytes + n * (1600 + 8 * BZ) + (PM == 3 && VM < 0 ? 1200 : 3700)); }
-    // 8-row tiles: up to three blocks of four warps; 16-row tiles: two blocks of four warps of 4-row
+    // 8-row tiles: up to three blocks of four warps, or the thin shape (kThinTiles); 16-row tiles: two blocks of four warps of 4-row
     // threads, or, where the stages are too large, one block of eight warps of 2-row threads
     static constexpr bool two = BZ == 16 && fit(2) >= 2;
-    static constexpr int U = BZ == 8 || (BZ == 16 && !two) ? 2 : BZ == 64 ? 8 : 4;
+    static constexpr int U = THIN ? 1 : BZ == 8 || (BZ == 16 && !two) ? 2 : BZ == 64 ? 8 : 4;
     static constexpr int warps = BZ / U, threads = 32 * (warps + 1);   // consumers; and the producer warp
-    static constexpr int blocks = BZ == 8 ? (PM == 3 && VM < 0 ? fit(2) : RTM_MIN2(fit(2), 3)) : two ? 2 : 1;
+    static constexpr int blocks = THIN ? 2 : BZ == 8 ? (PM == 3 && VM < 0 ? fit(2) : RTM_MIN2(fit(2), 3)) : two ? 2 : 1;
     static constexpr int stages = BZ <= 16 && blocks > 1 ? 2 : fit(3) ? 3 : fit(2) ? 2 : 1;
 };
 
@@ -208,45 +210,75 @@ __device__ __forceinline__ void fill_damping(StageMeta<BZ> &m, int c1x, int ic2x
     bulk_copy(m.c1z, pml + c1z + m.t.z0, BZ, bar);
     bulk_copy(m.ic2z, pml + ic2z + m.t.z0, BZ, bar);
 }
-// One thread: copy a tile's boxes into a stage.
+// One thread: the copies of a tile into a stage, in two parts: what no kernel of the pass writes (the
+// bytes expected in all, 1/rho or kappa, damping factors), which the first tile's copies can start
+// with before the kernel in front has finished, and the fields.
+template <int BZ, int MODE>
+__device__ __forceinline__ void fill_vel_const(StageMeta<BZ> &m, float *st, unsigned long long *bar)
+{
+    mbar_expect_tx(bar, ((BZ + 19) * WW + 3 * BZ * BX) * 4);
+    tma_box(st + Stage<BZ>::v_op, tmap_of(m.S, MODE == 0 ? RTM_TMAP_IRF : MODE == 2 ? RTM_TMAP_IRB : RTM_TMAP_IRB_RECON),
+            m.t.x0, m.t.z0, bar);
+    if (MODE != 3 && !(m.t.interior & 1)) {
+        const PmlOffsets o = pml_offsets(m.S.X, m.S.Z);
+        fill_damping<BZ>(m, o.c1vx, o.ic2vx, o.c1vz, o.ic2vz, bar);
+    }
+}
 template <int BZ, int MODE>
 __device__ __forceinline__ void fill_vel(const ShotDev &S, const TileRef &t, float *st, unsigned long long *bar)
 {
-    mbar_expect_tx(bar, ((BZ + 19) * WW + 3 * BZ * BX) * 4);
     float *op = st + Stage<BZ>::v_op;
     tma_box(st, tmap_of(S, MODE == 2 ? RTM_TMAP_B_P : MODE == 3 ? RTM_TMAP_A_P_RECON : RTM_TMAP_A_P), t.x0 - 12,
             t.z0 - 9, bar);
-    tma_box(op, tmap_of(S, MODE == 0 ? RTM_TMAP_IRF : MODE == 2 ? RTM_TMAP_IRB : RTM_TMAP_IRB_RECON), t.x0, t.z0, bar);
     tma_box(op + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_VX_OWN : MODE == 2 ? RTM_TMAP_B_VX_OWN : RTM_TMAP_A_VX_OWN_RECON),
             t.x0, t.z0, bar);
     tma_box(op + 2 * BZ * BX,
             tmap_of(S, MODE == 0 ? RTM_TMAP_A_VZ_OWN : MODE == 2 ? RTM_TMAP_B_VZ_OWN : RTM_TMAP_A_VZ_OWN_RECON), t.x0, t.z0,
             bar);
 }
+// What a pressure tile stages besides its boxes: imaging operands, or split fields.
+template <int BZ, int MODE>
+__device__ __forceinline__ bool stages_img(const TileRef &t)
+{
+    return BZ <= 16 && MODE == 2 && (t.interior & (1 | RTM_TILE_IMG));
+}
+template <int BZ, int MODE>
+__device__ __forceinline__ bool stages_band(const TileRef &t)
+{
+    return BZ <= 16 && MODE != 3 && (t.interior & RTM_TILE_BAND) && !stages_img<BZ, MODE>(t);
+}
+template <int BZ, int MODE, typename ACC>
+__device__ __forceinline__ void fill_pres_const(StageMeta<BZ> &m, float *st, unsigned long long *bar)
+{
+    constexpr int row = BZ * BX * 4;
+    mbar_expect_tx(bar, (BZ * WW + (BZ + 19) * BX) * 4 + 2 * row +
+                            (stages_img<BZ, MODE>(m.t) ? (1 + 2 * (int)sizeof(ACC) / 4) * row
+                             : stages_band<BZ, MODE>(m.t) ? 2 * row : 0));
+    tma_box(st + Stage<BZ>::p_op, tmap_of(m.S, MODE == 0 ? RTM_TMAP_KF : MODE == 2 ? RTM_TMAP_KB : RTM_TMAP_KB_RECON),
+            m.t.x0, m.t.z0, bar);
+    if (MODE != 3 && !(m.t.interior & 1)) {
+        const PmlOffsets o = pml_offsets(m.S.X, m.S.Z);
+        fill_damping<BZ>(m, o.c1x, o.ic2x, o.c1z, o.ic2z, bar);
+    }
+}
 template <int BZ, int MODE, typename ACC>
 __device__ __forceinline__ void fill_pres(const ShotDev &S, const TileRef &t, float *st, unsigned long long *bar)
 {
-    using P = Pipe<BZ, MODE, -1, ACC>;
-    const bool img = P::staged && MODE == 2 && (t.interior & (1 | RTM_TILE_IMG));
-    const bool band = P::staged && MODE != 3 && (t.interior & RTM_TILE_BAND) && !img;
-    mbar_expect_tx(bar, (BZ * WW + (BZ + 19) * BX + 2 * BZ * BX) * 4 +
-                            (img ? (1 + 2 * (int)sizeof(ACC) / 4) * P::row : band ? 2 * P::row : 0));
     tma_box(st, tmap_of(S, MODE == 2 ? RTM_TMAP_B_VX : MODE == 3 ? RTM_TMAP_A_VX_RECON : RTM_TMAP_A_VX), t.x0 - 12, t.z0,
             bar);
     tma_box(st + Stage<BZ>::p_vz, tmap_of(S, MODE == 2 ? RTM_TMAP_B_VZ : MODE == 3 ? RTM_TMAP_A_VZ_RECON : RTM_TMAP_A_VZ),
             t.x0, t.z0 - 10, bar);
     float *op = st + Stage<BZ>::p_op;
-    tma_box(op, tmap_of(S, MODE == 0 ? RTM_TMAP_KF : MODE == 2 ? RTM_TMAP_KB : RTM_TMAP_KB_RECON), t.x0, t.z0, bar);
     tma_box(op + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_P_OWN : MODE == 2 ? RTM_TMAP_B_P_OWN : RTM_TMAP_A_P_OWN_RECON),
             t.x0, t.z0, bar);
     float *ex = op + 2 * BZ * BX;
-    if (img) {   // ps, g1, illum (8-byte accumulators: two words per column)
+    if (stages_img<BZ, MODE>(t)) {   // ps, g1, illum (8-byte accumulators: two words per column)
         constexpr int w = (int)sizeof(ACC) / 4;
         tma_box(ex, tmap_of(S, RTM_TMAP_A_P_OWN), t.x0, t.z0, bar);
         tma_box(ex + BZ * BX, tmap_of(S, RTM_TMAP_G1), w * t.x0, t.z0, bar);
         tma_box(ex + (1 + w) * BZ * BX, tmap_of(S, RTM_TMAP_ILLUM), w * t.x0, t.z0, bar);
     }
-    if (band) {
+    if (stages_band<BZ, MODE>(t)) {
         tma_box(ex, tmap_of(S, MODE == 0 ? RTM_TMAP_A_SX : RTM_TMAP_B_SX), t.x0, t.z0, bar);
         tma_box(ex + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_SZ : RTM_TMAP_B_SZ), t.x0, t.z0, bar);
     }
@@ -338,8 +370,8 @@ __device__ __forceinline__ void vel_compute(const StepArgs &a, const StageMeta<B
     // vx order per column (cuda_norderx), vz order per row (cuda_norderz); the reconstruction
     // writes only cells at least npml >= R from the edge, where every order is full
     const auto order = [&](int i, int n) { return min(min(i + 1, n - 1 - i), R); };
-    const bool edge_x = MODE != 3 && (F & RTM_TILE_XEDGE);
-    const bool edge_z = MODE != 3 && (zr < R || zr + U > Z - R);
+    const bool edge_x = MODE != 3 && (U == 1 || (F & RTM_TILE_XEDGE));
+    const bool edge_z = MODE != 3 && (U == 1 || (zr < R || zr + U > Z - R));
     const float2 *ex[2] = {s_tab, s_tab};
     if (edge_x) {
         ex[0] = pair_row(s_tab, order(x, X), order(x + 1, X));
@@ -543,7 +575,7 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
     // local order of a cell (cuda_norder): the distance to the nearest edge in x or z, at most
     // R; 0 on the edge itself, which keeps its pressure
     const auto order = [&](int xj, int z) { return min(min(min(xj, X - 1 - xj), min(z, Z - 1 - z)), R); };
-    const bool edge = MODE != 3 && ((F & RTM_TILE_XEDGE) || zr < R || zr + U > Z - R);
+    const bool edge = MODE != 3 && (U == 1 || (F & RTM_TILE_XEDGE) || zr < R || zr + U > Z - R);
     const float2 *ec[U][2];   // edge groups: the coefficients of the row's two column pairs
     if (edge) {
 #pragma unroll
@@ -676,11 +708,11 @@ __device__ __forceinline__ void mbar_init_n(unsigned long long *bar, unsigned n)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
 
-template <int BZ, int PM, int VM, typename ACC>
-__global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC>::threads, Pipe<BZ, PM, VM, ACC>::blocks)
+template <int BZ, int PM, int VM, typename ACC, bool THIN>
+__global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ, PM, VM, ACC, THIN>::blocks)
     k_pipe(const StepArgs a, int ntiles, int record)
 {
-    using P = Pipe<BZ, PM, VM, ACC>;
+    using P = Pipe<BZ, PM, VM, ACC, THIN>;
     constexpr int ST = P::stages, U = P::U, SB = P::bytes, NC = P::warps;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(16) StageMeta<BZ> s_meta[ST];
@@ -720,11 +752,31 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC>::threads, Pipe<BZ, PM, V
             for (int k = 0; k < WL; k++) w[k] = lane + 32 * k < W ? src[lane + 32 * k] : 0u;
         };
         int i = blockIdx.x, ahead = i + step;
-        if (i < n) load(i);
+        // into stage s: the loaded tile's descriptor and its constant part
+        const auto begin = [&](int s) {
+            StageMeta<BZ> &m = s_meta[s];
+            unsigned *dst = (unsigned *)&m.S;
+#pragma unroll
+            for (int k = 0; k < WL; k++)
+                if (lane + 32 * k < W) dst[lane + 32 * k] = w[k];
+            if (lane == 0) m.t = t;
+            __syncwarp();
+            if (lane == 0) {
+                float *st = (float *)(smem + s * SB);
+                if (is_pres(t)) {
+                    if constexpr (PM >= 0) fill_pres_const<BZ, PM, ACC>(m, st, &s_full[s]);
+                } else {
+                    if constexpr (VM >= 0) fill_vel_const<BZ, VM>(m, st, &s_full[s]);
+                }
+            }
+        };
+        if (i < n) {
+            load(i);
+            begin(0);
+        }
         pdl_wait();
         if (blockIdx.x == 0 && lane == 0) a.queue[a.qsel ^ 1] = 0u;   // (the launch before has finished with it)
         const auto claim = [&] { return lane == 0 ? step + (int)atomicAdd(&a.queue[a.qsel], 1u) : 0; };
-        if (dynamic) ahead = claim();
         int s = 0;
         unsigned parity = 1;   // the first use of a stage waits for no one
         for (int k = 0;; k++) {   // k: stages filled so far
@@ -741,24 +793,12 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC>::threads, Pipe<BZ, PM, V
                 }
                 return;
             }
-            StageMeta<BZ> &m = s_meta[s];
-            unsigned *dst = (unsigned *)&m.S;
-#pragma unroll
-            for (int k = 0; k < WL; k++)
-                if (lane + 32 * k < W) dst[lane + 32 * k] = w[k];
-            if (lane == 0) m.t = t;
-            __syncwarp();
-            const ShotDev &S = m.S;
+            if (k > 0) begin(s);
+            const ShotDev &S = s_meta[s].S;
             float *st = (float *)(smem + s * SB);
             if (is_pres(t)) {
                 if constexpr (PM >= 0) {
-                    if (lane == 0) {
-                        fill_pres<BZ, PM, ACC>(S, t, st, &s_full[s]);
-                        if (PM != 3 && !(t.interior & 1)) {
-                            const PmlOffsets o = pml_offsets(S.X, S.Z);
-                            fill_damping<BZ>(m, o.c1x, o.ic2x, o.c1z, o.ic2z, &s_full[s]);
-                        }
-                    }
+                    if (lane == 0) fill_pres<BZ, PM, ACC>(S, t, st, &s_full[s]);
                     if (a.prefetch && PM != 3) {
                         const WaveDev &W_ = PM == 2 ? S.b : S.a;
                         const int z1 = min(t.z0 + BZ, S.Z);
@@ -776,14 +816,9 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC>::threads, Pipe<BZ, PM, V
                 }
             } else {
                 if constexpr (VM >= 0)
-                    if (lane == 0) {
-                        fill_vel<BZ, VM>(S, t, st, &s_full[s]);
-                        if (VM != 3 && !(t.interior & 1)) {
-                            const PmlOffsets o = pml_offsets(S.X, S.Z);
-                            fill_damping<BZ>(m, o.c1vx, o.ic2vx, o.c1vz, o.ic2vz, &s_full[s]);
-                        }
-                    }
+                    if (lane == 0) fill_vel<BZ, VM>(S, t, st, &s_full[s]);
             }
+            if (k == 0 && dynamic) ahead = claim();
             if (lane == 0) mbar_arrive(&s_full[s]);
             i = __shfl_sync(0xffffffffu, ahead, 0);
             if (i < n) {
@@ -820,10 +855,10 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC>::threads, Pipe<BZ, PM, V
 }
 
 // ---- host launchers ---------------------------------------------------------------------
-template <int BZ, int PM, int VM, typename ACC>
-void pipe_launch_t(const StepArgs &a, int ntiles, int record, cudaStream_t st)
+template <int BZ, int PM, int VM, typename ACC, bool THIN>
+void pipe_launch_v(const StepArgs &a, int ntiles, int record, cudaStream_t st)
 {
-    using P = Pipe<BZ, PM, VM, ACC>;
+    using P = Pipe<BZ, PM, VM, ACC, THIN>;
     constexpr size_t bytes = (size_t)P::stages * P::bytes;
     // the shared-memory limit is an attribute of the instance on each device; the resident
     // blocks per device follow from it (looked up once per device)
@@ -833,9 +868,9 @@ void pipe_launch_t(const StepArgs &a, int ntiles, int record, cudaStream_t st)
     int cap = dev < 64 ? slots[dev].load(std::memory_order_acquire) : 0;
     if (!cap) {
         int sms = 0, per = 0;
-        cudaFuncSetAttribute(k_pipe<BZ, PM, VM, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        cudaFuncSetAttribute(k_pipe<BZ, PM, VM, ACC, THIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pipe<BZ, PM, VM, ACC>, P::threads, bytes);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pipe<BZ, PM, VM, ACC, THIN>, P::threads, bytes);
         cap = sms * (per > 0 ? per : 1);
         if (dev < 64) slots[dev].store(cap, std::memory_order_release);
     }
@@ -849,7 +884,22 @@ void pipe_launch_t(const StepArgs &a, int ntiles, int record, cudaStream_t st)
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_pipe<BZ, PM, VM, ACC>, a, ntiles, record);
+    cudaLaunchKernelEx(&cfg, k_pipe<BZ, PM, VM, ACC, THIN>, a, ntiles, record);
+}
+
+// The 8-row tiles' launches of up to two tiles per SM take the thin shape (one row per thread, 8
+// consumer warps): every tile is then resident at once and a launch lasts as long as one tile's
+// chain of wait, sums and stores, which is shorter with half the rows per thread. A step of
+// 401x201 (248 tiles per launch) 21.7 us with U = 2 and 19.0 us thin, 201x101 20.2 and 18.4 us;
+// with more tiles than that the wide shape's fewer instructions and shared-memory reads per cell
+// count: 1701x351 at any length 36.1 us wide and 39.8 thin, 12 shots of 481x331 104.6 and 118.6 us.
+constexpr int kThinTiles = 296;
+template <int BZ, int PM, int VM, typename ACC>
+void pipe_launch_t(const StepArgs &a, int ntiles, int record, cudaStream_t st)
+{
+    if constexpr (BZ == 8)
+        if (ntiles <= kThinTiles) return pipe_launch_v<BZ, PM, VM, ACC, true>(a, ntiles, record, st);
+    pipe_launch_v<BZ, PM, VM, ACC, false>(a, ntiles, record, st);
 }
 
 }  // namespace

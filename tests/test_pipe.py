@@ -81,6 +81,20 @@ def test_pipelined_form_for_short_and_long_tile_lists(rtmlib, monkeypatch, shots
     _same(*_both(monkeypatch, G, heights, lambda: G.migrate(s, G.RunOptions(), list(range(1, shots + 1)), v, rho)))
 
 
+# 8-row tiles either side of the length up to which a launch takes one row per thread: 294 and 300
+# tiles in a merged launch, 147 and 150 in one kernel's
+@pytest.mark.gpu
+@pytest.mark.parametrize("Z", [392, 400])
+@pytest.mark.parametrize("accum", [0, 1, 2])
+@pytest.mark.parametrize("heights", [(8, 8, 8, 8), (16, 8, 8, 16)])
+def test_pipelined_form_of_eight_rows_either_side_of_two_tiles_per_sm(rtmlib, monkeypatch, Z, accum, heights):
+    G = rtmlib
+    nx, nz, npml = 344, Z - 40, 20
+    v, rho = _models(nz, nx, Z)
+    s = _survey(G, nx, nz, npml, 60, receiver_depth=2)
+    _same(*_both(monkeypatch, G, heights, lambda: G.migrate(s, G.RunOptions(accum_fp64=accum), [1], v, rho)))
+
+
 # chunk boundaries of the host copies: images of one chunk (2^18 floats), one cell less and more,
 # a small one and several chunks; fp64 images narrowed on the way; fields with row pitch
 @pytest.mark.gpu
