@@ -141,7 +141,6 @@ struct rtm_session {
     // pressure, reconstruction pressure): the pipelined one (rtm_pipe.cu) or one tile per block with
     // one column per thread (rtm_stencil.cu), by RTM_B200_KERNELS=vector|scalar
     bool vec[4] = {true, true, true, true};
-    bool forms_fixed = false;
     // backward pass in two merged launches per step (chosen by the tuner; needs every family in the
     // pipelined form at one tile height)
     bool merge = true;
@@ -504,7 +503,6 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
             if (std::strcmp(e, "scalar") && std::strcmp(e, "vector"))
                 return fail(RTM_ERR_ARG, "RTM_B200_KERNELS must be scalar or vector");
             for (bool &v : ss->vec) v = !std::strcmp(e, "vector");
-            ss->forms_fixed = true;
         }
         if (ss->persist) {   // the persistent passes run the one-column kernels at the default heights
             ss->tune = false;
@@ -516,7 +514,8 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
         if (o.extra_images < 0 || o.extra_images > 2) return fail(RTM_ERR_ARG, "extra_images must be 0, 1 or 2");
         if (o.accum_fp64 < 0 || o.accum_fp64 > 3) return fail(RTM_ERR_ARG, "accum_fp64 must be 0, 1, 2 or 3");
         for (int bz : {ss->bz_vel, ss->bz_vel_recon, ss->bz_pres, ss->bz_pres_recon})
-            if (bz != 8 && bz != 16 && bz != 32 && bz != 64) return fail(RTM_ERR_ARG, "tile heights must be 8, 16, 32 or 64");
+            if (bz != 8 && bz != 16 && bz != 32 && bz != 64 && !(bz == 12 && ss->vec[0]))
+                return fail(RTM_ERR_ARG, "tile heights must be 8, 16, 32 or 64 (or 12 in the pipelined form)");
     }
     B = std::max(B, 1);
     ss->B = B;
@@ -1758,7 +1757,7 @@ static int tune_heights(rtm_session *ss, int k0, int n)
         }
     }
     if (ss->fused) return tune_step_height(ss, k0, n, key, path);
-    const int cand[3] = {8, 16, 32}, nc = 3;   // tile heights
+    const int nc = ss->vec[0] ? 4 : 3, cand[4] = {8, 16, 32, 12};   // tile heights
     ss->merge = false;
     const char *names[6] = {"vel_fwd", "pres_fwd", "vel_recon", "pres_recon", "vel_recv", "pres_recv"};
     std::vector<std::array<double, 6>> ms(nc, std::array<double, 6>{});
@@ -1841,6 +1840,10 @@ static int tune_heights(rtm_session *ss, int k0, int n)
     };
     std::vector<Plan> plans = {{best, false, 0.f}};
     if (ss->vec[0] && !ss->o.extra_images) {
+        // (a kernel's time alone leaves out how its blocks start beside those of the launch before:
+        // 64 shots of 1801x451 at 16/8/12/8 1384 us a step, at 16/16/12/8 1300, although velocity
+        // reconstruction alone takes 171 us at either height)
+        if (best[1] != best[0]) plans.push_back({{best[0], best[0], best[2], best[3]}, false, 0.f});
         plans.push_back({{8, 8, 8, 8}, true, 0.f});
         plans.push_back({{16, 16, 16, 16}, true, 0.f});
         cudaEvent_t e0, e1;

@@ -12,6 +12,7 @@ void launch_pres(int mode, int bz, const StepArgs &a, int ntiles, int record, cu
 // of that kind; both: a merged list whose velocity tiles carry RTM_TILE_VEL): same results.
 // One translation unit per tile height.
 void launch_pipe_8(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
+void launch_pipe_12(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
 void launch_pipe_16(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
 void launch_pipe_32(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
 void launch_pipe_64(int pm, int vm, const StepArgs &a, int ntiles, int record, cudaStream_t s);
@@ -19,6 +20,7 @@ inline void launch_pipe(int pm, int vm, int bz, const StepArgs &a, int ntiles, i
 {
     if (bz == 16) launch_pipe_16(pm, vm, a, ntiles, record, s);
     else if (bz == 8) launch_pipe_8(pm, vm, a, ntiles, record, s);
+    else if (bz == 12) launch_pipe_12(pm, vm, a, ntiles, record, s);
     else if (bz == 64) launch_pipe_64(pm, vm, a, ntiles, record, s);
     else launch_pipe_32(pm, vm, a, ntiles, record, s);
 }

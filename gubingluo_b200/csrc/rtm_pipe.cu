@@ -166,10 +166,15 @@ struct Pipe {
     // blocks of n stages that fit an SM's shared memory (a block's own part: descriptors, barriers,
     // coefficients and the system's 1 KB)
     static constexpr int fit(int n) { return 228 * 1024 / (n * bytes + n * (1600 + 8 * BZ) + (PM == 3 && VM < 0 ? 1200 : 3700)); }
-    // 8-row tiles: up to three blocks of four warps, or the thin shape (kThinTiles); 16-row tiles: two blocks of four warps of 4-row
-    // threads, or, where the stages are too large, one block of eight warps of 2-row threads
-    static constexpr bool two = BZ == 16 && fit(2) >= 2;
-    static constexpr int U = THIN ? 1 : BZ == 8 || (BZ == 16 && !two) ? 2 : BZ == 64 ? 8 : 4;
+    // 8-row tiles: up to three blocks of four warps, or the thin shape (kThinTiles).  12- and 16-row
+    // tiles: two blocks where two stages each fit, else one.  The rows a thread takes: fewer rows mean
+    // more shared-memory reads per cell but twice the warps, and with eight consumer warps on an SM
+    // the pressure kernels wait on instruction and read latency (issue slots 34% used, DRAM 46%):
+    // 64 shots of 1801x451 (us, 12 rows with U = 3 / 2) forward pressure 306 / 276, receiver pressure
+    // 320 / 328; a step of 16 shots 389 / 370.  Velocity at 16 rows reads the least per cell and is
+    // at the memory's rate with U = 4: 203 / 221 (U = 4 / 2).
+    static constexpr bool two = (BZ == 12 || BZ == 16) && fit(2) >= 2;
+    static constexpr int U = THIN ? 1 : BZ == 16 ? (PM < 0 ? 4 : 2) : BZ <= 12 ? 2 : BZ == 64 ? 8 : 4;
     static constexpr int warps = BZ / U, threads = 32 * (warps + 1);   // consumers; and the producer warp
     static constexpr int blocks = THIN ? 2 : BZ == 8 ? (PM == 3 && VM < 0 ? fit(2) : RTM_MIN2(fit(2), 3)) : two ? 2 : 1;
     static constexpr int stages = BZ <= 16 && blocks > 1 ? 2 : fit(3) ? 3 : fit(2) ? 2 : 1;
@@ -210,9 +215,13 @@ __device__ __forceinline__ void fill_damping(StageMeta<BZ> &m, int c1x, int ic2x
     bulk_copy(m.c1z, pml + c1z + m.t.z0, BZ, bar);
     bulk_copy(m.ic2z, pml + ic2z + m.t.z0, BZ, bar);
 }
+__device__ __forceinline__ const void *tmap(const char *maps, int which) { return maps + which * RTM_TMAP_BYTES; }
 // One thread: the copies of a tile into a stage, in two parts: what no kernel of the pass writes (the
-// bytes expected in all, 1/rho or kappa, damping factors), which the first tile's copies can start
-// with before the kernel in front has finished, and the fields.
+// bytes expected in all, 1/rho or kappa, damping factors), which the first tile's copies start with
+// before the kernel in front has finished, and the fields, which come first in every later tile:
+// a stage is idle until its largest boxes are on their way (64 shots of 1801x451: 1369 us a step
+// with the constant part first, 1324 with the fields first, 1300 with the descriptor's words
+// stored after the fields' copies too).
 template <int BZ, int MODE>
 __device__ __forceinline__ void fill_vel_const(StageMeta<BZ> &m, float *st, unsigned long long *bar)
 {
@@ -225,15 +234,15 @@ __device__ __forceinline__ void fill_vel_const(StageMeta<BZ> &m, float *st, unsi
     }
 }
 template <int BZ, int MODE>
-__device__ __forceinline__ void fill_vel(const ShotDev &S, const TileRef &t, float *st, unsigned long long *bar)
+__device__ __forceinline__ void fill_vel(const char *maps, const TileRef &t, float *st, unsigned long long *bar)
 {
     float *op = st + Stage<BZ>::v_op;
-    tma_box(st, tmap_of(S, MODE == 2 ? RTM_TMAP_B_P : MODE == 3 ? RTM_TMAP_A_P_RECON : RTM_TMAP_A_P), t.x0 - 12,
+    tma_box(st, tmap(maps, MODE == 2 ? RTM_TMAP_B_P : MODE == 3 ? RTM_TMAP_A_P_RECON : RTM_TMAP_A_P), t.x0 - 12,
             t.z0 - 9, bar);
-    tma_box(op + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_VX_OWN : MODE == 2 ? RTM_TMAP_B_VX_OWN : RTM_TMAP_A_VX_OWN_RECON),
+    tma_box(op + BZ * BX, tmap(maps, MODE == 0 ? RTM_TMAP_A_VX_OWN : MODE == 2 ? RTM_TMAP_B_VX_OWN : RTM_TMAP_A_VX_OWN_RECON),
             t.x0, t.z0, bar);
     tma_box(op + 2 * BZ * BX,
-            tmap_of(S, MODE == 0 ? RTM_TMAP_A_VZ_OWN : MODE == 2 ? RTM_TMAP_B_VZ_OWN : RTM_TMAP_A_VZ_OWN_RECON), t.x0, t.z0,
+            tmap(maps, MODE == 0 ? RTM_TMAP_A_VZ_OWN : MODE == 2 ? RTM_TMAP_B_VZ_OWN : RTM_TMAP_A_VZ_OWN_RECON), t.x0, t.z0,
             bar);
 }
 // What a pressure tile stages besides its boxes: imaging operands, or split fields.
@@ -262,25 +271,25 @@ __device__ __forceinline__ void fill_pres_const(StageMeta<BZ> &m, float *st, uns
     }
 }
 template <int BZ, int MODE, typename ACC>
-__device__ __forceinline__ void fill_pres(const ShotDev &S, const TileRef &t, float *st, unsigned long long *bar)
+__device__ __forceinline__ void fill_pres(const char *maps, const TileRef &t, float *st, unsigned long long *bar)
 {
-    tma_box(st, tmap_of(S, MODE == 2 ? RTM_TMAP_B_VX : MODE == 3 ? RTM_TMAP_A_VX_RECON : RTM_TMAP_A_VX), t.x0 - 12, t.z0,
+    tma_box(st, tmap(maps, MODE == 2 ? RTM_TMAP_B_VX : MODE == 3 ? RTM_TMAP_A_VX_RECON : RTM_TMAP_A_VX), t.x0 - 12, t.z0,
             bar);
-    tma_box(st + Stage<BZ>::p_vz, tmap_of(S, MODE == 2 ? RTM_TMAP_B_VZ : MODE == 3 ? RTM_TMAP_A_VZ_RECON : RTM_TMAP_A_VZ),
+    tma_box(st + Stage<BZ>::p_vz, tmap(maps, MODE == 2 ? RTM_TMAP_B_VZ : MODE == 3 ? RTM_TMAP_A_VZ_RECON : RTM_TMAP_A_VZ),
             t.x0, t.z0 - 10, bar);
     float *op = st + Stage<BZ>::p_op;
-    tma_box(op + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_P_OWN : MODE == 2 ? RTM_TMAP_B_P_OWN : RTM_TMAP_A_P_OWN_RECON),
+    tma_box(op + BZ * BX, tmap(maps, MODE == 0 ? RTM_TMAP_A_P_OWN : MODE == 2 ? RTM_TMAP_B_P_OWN : RTM_TMAP_A_P_OWN_RECON),
             t.x0, t.z0, bar);
     float *ex = op + 2 * BZ * BX;
     if (stages_img<BZ, MODE>(t)) {   // ps, g1, illum (8-byte accumulators: two words per column)
         constexpr int w = (int)sizeof(ACC) / 4;
-        tma_box(ex, tmap_of(S, RTM_TMAP_A_P_OWN), t.x0, t.z0, bar);
-        tma_box(ex + BZ * BX, tmap_of(S, RTM_TMAP_G1), w * t.x0, t.z0, bar);
-        tma_box(ex + (1 + w) * BZ * BX, tmap_of(S, RTM_TMAP_ILLUM), w * t.x0, t.z0, bar);
+        tma_box(ex, tmap(maps, RTM_TMAP_A_P_OWN), t.x0, t.z0, bar);
+        tma_box(ex + BZ * BX, tmap(maps, RTM_TMAP_G1), w * t.x0, t.z0, bar);
+        tma_box(ex + (1 + w) * BZ * BX, tmap(maps, RTM_TMAP_ILLUM), w * t.x0, t.z0, bar);
     }
     if (stages_band<BZ, MODE>(t)) {
-        tma_box(ex, tmap_of(S, MODE == 0 ? RTM_TMAP_A_SX : RTM_TMAP_B_SX), t.x0, t.z0, bar);
-        tma_box(ex + BZ * BX, tmap_of(S, MODE == 0 ? RTM_TMAP_A_SZ : RTM_TMAP_B_SZ), t.x0, t.z0, bar);
+        tma_box(ex, tmap(maps, MODE == 0 ? RTM_TMAP_A_SX : RTM_TMAP_B_SX), t.x0, t.z0, bar);
+        tma_box(ex + BZ * BX, tmap(maps, MODE == 0 ? RTM_TMAP_A_SZ : RTM_TMAP_B_SZ), t.x0, t.z0, bar);
     }
 }
 
@@ -317,7 +326,32 @@ __device__ __forceinline__ float *strip_dst(const StepArgs &a, const ShotDev &S)
                                     : S.strip_stage + (size_t)a.ring * S.strip_len;
 }
 
-// ---- velocity (later: the step whose saved strips the reconstruction restores) ---------------------------------------------------------------------------
+// The columns of a word that lie in a strip (mask m): saved to d[0 .. 3], restored from i0 .. i0+3.
+__device__ __forceinline__ void strip_put(float *d, unsigned m, const float (&v)[4])
+{
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (m >> j & 1) d[j] = v[j];
+}
+__device__ __forceinline__ void strip_get(float (&v)[4], const void *strips, size_t i0, unsigned m, int prec, float scale)
+{
+    if (prec == RTM_FP32) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (m >> j & 1) v[j] = ((const float *)strips + i0)[j];
+        return;
+    }
+    const unsigned short *p = (const unsigned short *)strips + i0;
+    unsigned short h[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (m >> j & 1) h[j] = p[j];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        v[j] = (prec == RTM_FP16 ? __half2float(__ushort_as_half(h[j])) : __bfloat162float(__ushort_as_bfloat16(h[j]))) * scale;
+}
+
+// ---- velocity (later: the step whose saved strips the reconstruction restores) -----------
 template <int BZ, int U, int MODE>
 __device__ __forceinline__ void vel_compute(const StepArgs &a, const StageMeta<BZ> &m, const TileRef &t, const float *st,
                                             const float2 *s_tab, int later)
@@ -382,49 +416,55 @@ __device__ __forceinline__ void vel_compute(const StepArgs &a, const StageMeta<B
     else dz_sum<U, WW>(colbase, dz, [&](int u, int, int i) { return s_tab[(max(order(zr + u, Z), 1) - 1) * R + i]; });
     const int nxi = S.nxi, nzi = S.nzi;
     const bool save = MODE == 0 && a.save;
+    // strip cells of column x in row zr: vx left and right of the interior (R apart per row), and vz
+    // in row 0 of its strips
+    const int sl = (zr - npml) * R + x - (npml - R), sr = (nzi + zr - npml) * R + x - (X - npml - 1);
+    const int stb = 2 * R * nzi + x - npml;
+    const unsigned mtb = MODE == 3 ? mvz : cols_in(x, npml, X - npml);
+    float *strips = save ? strip_dst(a, S) : nullptr;
+    const size_t s0 = (size_t)later * S.strip_len;
+    float scx = 1.0f, scz = 1.0f;
+    if (MODE == 3 && a.strip_prec) {
+        scx = S.strip_scale[(size_t)later * 4 + 0];
+        scz = S.strip_scale[(size_t)later * 4 + 1];
+    }
     unsigned id = (unsigned)zr * pitch + x;
 #pragma unroll
     for (int u = 0; u < U; u++, id += pitch) {
         const int z = zr + u;
         if (z >= Z) break;
+        const bool zin = z >= npml && z < Z - npml;
+        const int srow = MODE == 3 || save ? strip_row_tb(z, npml, Z - npml - 1, nxi) : -1;
+        float rx[4], rz[4];   // restored: vx of a row of the interior, vz of a strip row
+        if (MODE == 3 && zin) {   // read_d_vxpml, kernel.cu:1294-1320
+            if (msl) strip_get(rx, S.strips, s0 + sl + u * R, msl, a.strip_prec, scx);
+            if (msr) {
+                float q[4];
+                strip_get(q, S.strips, s0 + sr + u * R, msr, a.strip_prec, scx);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (msr >> j & 1) rx[j] = q[j];
+            }
+        }
+        if (MODE == 3 && srow >= 0 && mvz)   // read_d_vzpml, kernel.cu:1321-1347
+            strip_get(rz, S.strips, s0 + stb + srow, mvz, a.strip_prec, scz);
         P4 dx;
         if (!edge_x) dx = dx_sum<12, 13>(rowbase + u * WW, cx);
         else dx = dx_sum<12, 13>(rowbase + u * WW, [&](int h, int i) { return ex[h][i]; });
         const P4 ir = p4(lds4(op + u * BX));
         const P4 ix = mul(mul(dx, dtx), ir), iz = mul(mul(dz[u], dtz), ir);
         const float4 ov = lds4(op + (BZ + u) * BX), ow = lds4(op + (2 * BZ + u) * BX);
-        const bool zin = z >= npml && z < Z - npml;
         if (MODE == 3) {
             // kernel.cu:318-388 (+=) on the interior; strips of the step after elsewhere
-            const size_t s0 = (size_t)later * S.strip_len;
-            if (zin && (mvx | msl | msr)) {   // read_d_vxpml, kernel.cu:1294-1320
+            if (zin && (mvx | msl | msr)) {
                 float4 n = pick(mvx, q4(sub(p4(ov), ix)), ov);
-                if (msl | msr) {
-                    const float sc = a.strip_prec ? S.strip_scale[(size_t)later * 4 + 0] : 1.0f;
-                    float v[4] = {n.x, n.y, n.z, n.w};
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if ((msl | msr) >> j & 1) {
-                            const int c = msl >> j & 1 ? x + j - (npml - R) : R * nzi + x + j - (X - npml - 1);
-                            v[j] = load_strip(S.strips, s0 + c + (size_t)(z - npml) * R, a.strip_prec, sc);
-                        }
-                    n = f4(v);
-                }
+                if (msl | msr) n = pick(msl | msr, f4(rx), n);
                 st4(&vxp[id], n);
             }
             if (z >= npml && z <= Z - npml - 2) {
                 if (mvz) st4(&vzp[id], pick(mvz, q4(sub(p4(ow), iz)), ow));
-            } else if (mvz && z < Z - 1) {   // read_d_vzpml, kernel.cu:1321-1347
-                const int srow = strip_row_tb(z, npml, Z - npml - 1, nxi);
-                if (srow >= 0) {
-                    const float sc = a.strip_prec ? S.strip_scale[(size_t)later * 4 + 1] : 1.0f;
-                    float v[4] = {ow.x, ow.y, ow.z, ow.w};
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if (mvz >> j & 1)
-                            v[j] = load_strip(S.strips, s0 + 2 * (size_t)R * nzi + srow + (x + j - npml), a.strip_prec, sc);
-                    st4(&vzp[id], f4(v));
-                }
+            } else if (mvz && srow >= 0) {
+                st4(&vzp[id], pick(mvz, f4(rz), ow));
             }
             continue;
         }
@@ -444,21 +484,10 @@ __device__ __forceinline__ void vel_compute(const StepArgs &a, const StageMeta<B
         if (F & RTM_TILE_XBAND) nz = pick(mvz, nz, ow);
         st4(&vzp[id], nz);
         if (save) {   // save_d_vxpml, save_d_vzpml (kernel.cu:1186-1240)
-            if (zin && (msl | msr)) {
-                float *d = strip_dst(a, S) + (z - npml) * R;
-                const float v[4] = {nx.x, nx.y, nx.z, nx.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if ((msl | msr) >> j & 1) d[msl >> j & 1 ? x + j - (npml - R) : R * nzi + x + j - (X - npml - 1)] = v[j];
-            }
-            const int srow = strip_row_tb(z, npml, Z - npml - 1, nxi);
-            if (srow >= 0) {
-                float *d = strip_dst(a, S) + 2 * R * nzi + srow - npml;
-                const float v[4] = {nz.x, nz.y, nz.z, nz.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (x + j >= npml && x + j < X - npml) d[x + j] = v[j];
-            }
+            const float vx[4] = {nx.x, nx.y, nx.z, nx.w}, vz[4] = {nz.x, nz.y, nz.z, nz.w};
+            if (zin && msl) strip_put(strips + sl + u * R, msl, vx);
+            if (zin && msr) strip_put(strips + sr + u * R, msr, vx);
+            if (srow >= 0) strip_put(strips + stb + srow, mtb, vz);
         }
     }
 }
@@ -590,7 +619,17 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
     else dz_sum<U, BX>(colbase, dz, ecoef);
     const int nxi = S.nxi, nzi = S.nzi;
     const bool save = MODE == 0 && a.save;
-    const int ps0 = 2 * R * (nzi + nxi);   // first p strip
+    // strip cells of column x in row zr: p left and right of the interior (R apart per row), and in
+    // row 0 of the strips above and below it
+    const int ps0 = 2 * R * (nzi + nxi), sl = ps0 + (zr - npml) * R + x - (npml - R),
+              sr = ps0 + (nzi + zr - npml) * R + x - (X - npml), stb = ps0 + 2 * R * nzi + x - npml;
+    float *strips = save ? strip_dst(a, S) : nullptr;
+    const size_t s0 = (size_t)a.it * S.strip_len;
+    float scx = 1.0f, scz = 1.0f;
+    if (MODE == 3 && a.strip_prec) {
+        scx = S.strip_scale[(size_t)a.it * 4 + 2];
+        scz = S.strip_scale[(size_t)a.it * 4 + 3];
+    }
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const int z = zr + u;
@@ -598,6 +637,22 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
         const unsigned id = id0 + u * pitch;
         const int k = u & 1;
         if (u + 1 < U) load(u + 1);
+        const bool zin = z >= npml && z < Z - npml;
+        const int srow = (MODE == 3 || save) && !zin ? strip_row_tb(z, npml, Z - npml, nxi) : -1;
+        unsigned ml = 0u;   // restored columns
+        float rp[4];
+        if (MODE == 3) {   // read_d_ppmllr, read_d_ppmltb (kernel.cu:1348-1400)
+            ml = zin ? msl | msr : srow >= 0 ? min_ : 0u;
+            if (zin && msl) strip_get(rp, S.strips, s0 + sl + u * R, msl, a.strip_prec, scx);
+            if (zin && msr) {
+                float q[4];
+                strip_get(q, S.strips, s0 + sr + u * R, msr, a.strip_prec, scx);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (msr >> j & 1) rp[j] = q[j];
+            }
+            if (srow >= 0 && min_) strip_get(rp, S.strips, s0 + stb + srow, min_, a.strip_prec, scz);
+        }
         P4 dx;
         if (!edge) dx = dx_sum<11, 12>(rowbase + u * WW, cx);
         else dx = dx_sum<11, 12>(rowbase + u * WW, [&](int h, int i) { return ecoef(u, h, i); });
@@ -605,30 +660,15 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
         const float4 p0 = lds4(op + (BZ + u) * BX);
         const P4 dxs = mul(mul(dx, dtx), kk), mdzs = mul(mul(dz[u], mdtz), kk);
         const float4 inner = q4(sub(p4(p0), sub(dxs, mdzs)));
-        const bool zin = z >= npml && z < Z - npml;
         float pn[4];
         bool wr = true;
         if (MODE == 3) {
             // reconstruction: kernel.cu:389-429, strips of step it, source subtracted
             const unsigned up = zin ? min_ : 0u;
-            const float4 n = pick(up, inner, p0);
+            float4 n = pick(up, inner, p0);
+            if (ml) n = pick(ml, f4(rp), n);
             pn[0] = n.x; pn[1] = n.y; pn[2] = n.z; pn[3] = n.w;
-            wr = up != 0;
-            const size_t s0 = (size_t)a.it * S.strip_len + ps0;
-            const int srow = zin ? -1 : strip_row_tb(z, npml, Z - npml, nxi);
-            const unsigned ml = zin ? msl | msr : srow >= 0 ? min_ : 0u;   // read_d_ppmllr / _ppmltb, kernel.cu:1348-1400
-            if (ml) {
-                const float sc = a.strip_prec ? S.strip_scale[(size_t)a.it * 4 + (zin ? 2 : 3)] : 1.0f;
-                wr = true;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (ml >> j & 1) {
-                        const size_t c = !zin ? 2 * (size_t)R * nzi + srow + (x + j - npml)
-                                              : (size_t)(msl >> j & 1 ? x + j - (npml - R) : R * nzi + x + j - (X - npml)) +
-                                                    (size_t)(z - npml) * R;
-                        pn[j] = load_strip(S.strips, s0 + c, a.strip_prec, sc);
-                    }
-            }
+            wr = (up | ml) != 0;
         } else {
             // kernel.cu:501-541 (interior) and :714-1185 (split-field PML)
             const unsigned in = zin ? min_ : 0u;
@@ -681,19 +721,9 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
         if (wr) st4(&pp[id], f4(pn));
         if (MODE == 2 && zin && min_) image(u, f4(pn));
         if (save) {   // save_d_ppmllr, save_d_ppmltb (kernel.cu:1241-1293)
-            if (zin && (msl | msr)) {
-                float *d = strip_dst(a, S) + ps0 + (z - npml) * R;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if ((msl | msr) >> j & 1) d[msl >> j & 1 ? x + j - (npml - R) : R * nzi + x + j - (X - npml)] = pn[j];
-            }
-            const int srow = strip_row_tb(z, npml, Z - npml, nxi);
-            if (srow >= 0 && min_) {
-                float *d = strip_dst(a, S) + ps0 + 2 * R * nzi + srow - npml;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (min_ >> j & 1) d[x + j] = pn[j];
-            }
+            if (zin && msl) strip_put(strips + sl + u * R, msl, pn);
+            if (zin && msr) strip_put(strips + sr + u * R, msr, pn);
+            if (srow >= 0) strip_put(strips + stb + srow, min_, pn);
         }
     }
 }
@@ -744,7 +774,7 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
         const bool back = !dynamic && a.qsel;
         constexpr int W = sizeof(ShotDev) / 4, WL = (W + 31) / 32;
         TileRef t{};
-        unsigned w[WL];   // the next tile's shot descriptor, one word per lane and round
+        unsigned w[WL] = {};   // the next tile's shot descriptor, one word per lane and round
         const auto load = [&](int i) {
             t = a.tiles[back ? n - 1 - i : i];
             const unsigned *src = (const unsigned *)&a.shots[t.shot];
@@ -752,7 +782,7 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
             for (int k = 0; k < WL; k++) w[k] = lane + 32 * k < W ? src[lane + 32 * k] : 0u;
         };
         int i = blockIdx.x, ahead = i + step;
-        // into stage s: the loaded tile's descriptor and its constant part
+        // into stage s: the loaded tile's descriptor
         const auto begin = [&](int s) {
             StageMeta<BZ> &m = s_meta[s];
             unsigned *dst = (unsigned *)&m.S;
@@ -761,18 +791,17 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
                 if (lane + 32 * k < W) dst[lane + 32 * k] = w[k];
             if (lane == 0) m.t = t;
             __syncwarp();
-            if (lane == 0) {
-                float *st = (float *)(smem + s * SB);
-                if (is_pres(t)) {
-                    if constexpr (PM >= 0) fill_pres_const<BZ, PM, ACC>(m, st, &s_full[s]);
-                } else {
-                    if constexpr (VM >= 0) fill_vel_const<BZ, VM>(m, st, &s_full[s]);
-                }
-            }
         };
         if (i < n) {
             load(i);
             begin(0);
+            if (lane == 0) {
+                if (is_pres(t)) {
+                    if constexpr (PM >= 0) fill_pres_const<BZ, PM, ACC>(s_meta[0], (float *)smem, &s_full[0]);
+                } else {
+                    if constexpr (VM >= 0) fill_vel_const<BZ, VM>(s_meta[0], (float *)smem, &s_full[0]);
+                }
+            }
         }
         pdl_wait();
         if (blockIdx.x == 0 && lane == 0) a.queue[a.qsel ^ 1] = 0u;   // (the launch before has finished with it)
@@ -780,6 +809,10 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
         int s = 0;
         unsigned parity = 1;   // the first use of a stage waits for no one
         for (int k = 0;; k++) {   // k: stages filled so far
+            constexpr int M = offsetof(ShotDev, tmaps) / 4;   // (the shot's tensor maps, from the loaded words)
+            const unsigned m0 = __shfl_sync(0xffffffffu, w[M / 32], M % 32);
+            const unsigned m1 = __shfl_sync(0xffffffffu, w[(M + 1) / 32], (M + 1) % 32);
+            const char *maps = (const char *)((unsigned long long)m1 << 32 | m0);
             if (!tile_wait(&s_empty[s], a.err, parity)) {
                 // the consumers are gone: leave when the copies in flight have landed (bounded)
                 for (int q = 0; q < ST; q++)
@@ -793,12 +826,15 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
                 }
                 return;
             }
-            if (k > 0) begin(s);
-            const ShotDev &S = s_meta[s].S;
             float *st = (float *)(smem + s * SB);
             if (is_pres(t)) {
                 if constexpr (PM >= 0) {
-                    if (lane == 0) fill_pres<BZ, PM, ACC>(S, t, st, &s_full[s]);
+                    if (lane == 0) fill_pres<BZ, PM, ACC>(maps, t, st, &s_full[s]);
+                    if (k > 0) {
+                        begin(s);
+                        if (lane == 0) fill_pres_const<BZ, PM, ACC>(s_meta[s], st, &s_full[s]);
+                    }
+                    const ShotDev &S = s_meta[s].S;
                     if (a.prefetch && PM != 3) {
                         const WaveDev &W_ = PM == 2 ? S.b : S.a;
                         const int z1 = min(t.z0 + BZ, S.Z);
@@ -815,8 +851,13 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
                     }
                 }
             } else {
-                if constexpr (VM >= 0)
-                    if (lane == 0) fill_vel<BZ, VM>(S, t, st, &s_full[s]);
+                if constexpr (VM >= 0) {
+                    if (lane == 0) fill_vel<BZ, VM>(maps, t, st, &s_full[s]);
+                    if (k > 0) {
+                        begin(s);
+                        if (lane == 0) fill_vel_const<BZ, VM>(s_meta[s], st, &s_full[s]);
+                    }
+                }
             }
             if (k == 0 && dynamic) ahead = claim();
             if (lane == 0) mbar_arrive(&s_full[s]);
@@ -859,7 +900,15 @@ template <int BZ, int PM, int VM, typename ACC, bool THIN>
 void pipe_launch_v(const StepArgs &a, int ntiles, int record, cudaStream_t st)
 {
     using P = Pipe<BZ, PM, VM, ACC, THIN>;
-    constexpr size_t bytes = (size_t)P::stages * P::bytes;
+    // every launch of b blocks per SM takes a b-th of the SM's shared memory for each: a block of the
+    // next launch, which starts when a block of this one ends, then fits the room that it leaves (with
+    // each kernel's own size the rooms left over were too small for a third block, and a launch of
+    // 8-row tiles ran in two waves: modelling 64 shots of 1801x451 724 us a step, 524 without the
+    // early starts, 16 shots' migration 451 and, with equal rooms, 403)
+    constexpr size_t used = (size_t)P::stages * P::bytes;
+    constexpr size_t own = 1024 + P::stages * (sizeof(StageMeta<BZ>) + 16) + (PM == 3 && VM < 0 ? 0 : kPairs * sizeof(float2));
+    constexpr size_t room = (228 * 1024 / P::blocks - own) / 128 * 128;
+    constexpr size_t bytes = P::blocks > 1 && room > used ? room : used;
     // the shared-memory limit is an attribute of the instance on each device; the resident
     // blocks per device follow from it (looked up once per device)
     static std::atomic<int> slots[64];

@@ -70,7 +70,7 @@ struct PmlOffsets {
 __host__ __device__ inline PmlOffsets pml_offsets(int X, int Z)
 {
     PmlOffsets o;
-    const int PX = (X + RTM_BX - 1) / RTM_BX * RTM_BX, PZ = (Z + 63) / 64 * 64;
+    const int PX = (X + RTM_BX - 1) / RTM_BX * RTM_BX, PZ = (Z + 75) / 64 * 64;   // past the last tile's rows at every height
     o.c1x = 0; o.ic2x = PX; o.c1vx = 2 * PX; o.ic2vx = 3 * PX;
     o.c1z = 4 * PX; o.ic2z = 4 * PX + PZ; o.c1vz = 4 * PX + 2 * PZ; o.ic2vz = 4 * PX + 3 * PZ;
     o.ddx = 4 * PX + 4 * PZ; o.ddz = o.ddx + X; o.ddxvx = o.ddz + Z; o.ddzvz = o.ddxvx + X;

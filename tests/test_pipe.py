@@ -95,6 +95,46 @@ def test_pipelined_form_of_eight_rows_either_side_of_two_tiles_per_sm(rtmlib, mo
     _same(*_both(monkeypatch, G, heights, lambda: G.migrate(s, G.RunOptions(accum_fp64=accum), [1], v, rho)))
 
 
+# 12-row tiles, which the one-column kernels do not have: with every tile on the general body all
+# heights round alike; the interior body of the forward pressure fuses one product (compared with the
+# tolerance of test_gpu_parity, 1e-4).  Depths that leave 1, 8 and 11 rows in the last tile, padded
+# lengths at the end of the damping factors' padding (64 rows), both strip types and accumulators
+@pytest.mark.gpu
+@pytest.mark.parametrize("X,Z,npml,accum", [(384, 133, 20, 0), (513, 128, 21, 1), (400, 191, 10, 2), (60, 64, 12, 0),
+                                            (390, 320, 33, 3)])
+@pytest.mark.parametrize("heights", [(12, 12, 12, 12), (16, 16, 12, 8)])
+def test_pipelined_form_at_twelve_rows(rtmlib, monkeypatch, X, Z, npml, accum, heights):
+    G = rtmlib
+    nx, nz = X - 2 * npml, Z - 2 * npml
+    v, rho = _models(nz, nx, X + Z)
+    s = _survey(G, nx, nz, npml, 90)
+    o = G.RunOptions(accum_fp64=accum, strip_precision="fp16" if accum == 2 else "fp32")
+    run = lambda: G.migrate(s, o, [1, 3], v, rho)
+    monkeypatch.setenv("RTM_B200_FAST_TILES", "0")
+    monkeypatch.setenv("RTM_B200_KERNELS", "scalar")
+    for k in ("VEL", "VEL_RECON", "PRES", "PRES_RECON"):
+        monkeypatch.setenv("RTM_B200_BZ_" + k, "16")
+    want = run()
+    monkeypatch.setenv("RTM_B200_KERNELS", "vector")
+    for k, h in zip(("VEL", "VEL_RECON", "PRES", "PRES_RECON"), heights):
+        monkeypatch.setenv("RTM_B200_BZ_" + k, str(h))
+    _same(want, run())
+    monkeypatch.delenv("RTM_B200_FAST_TILES")
+    got = run()
+    for k in ("image1", "image2s", "illum"):
+        a, b = got[k].astype(np.float64), want[k].astype(np.float64)
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b), k
+
+
+@pytest.mark.gpu
+def test_twelve_rows_need_the_pipelined_form(rtmlib, monkeypatch):
+    v, rho = _models(60, 60, 0)
+    monkeypatch.setenv("RTM_B200_KERNELS", "scalar")
+    monkeypatch.setenv("RTM_B200_BZ_PRES", "12")
+    with pytest.raises(rtmlib.RtmError):
+        rtmlib.migrate(_survey(rtmlib, 60, 60, 12, 30), rtmlib.RunOptions(), [1], v, rho)
+
+
 # chunk boundaries of the host copies: images of one chunk (2^18 floats), one cell less and more,
 # a small one and several chunks; fp64 images narrowed on the way; fields with row pitch
 @pytest.mark.gpu
