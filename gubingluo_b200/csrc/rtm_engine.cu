@@ -486,6 +486,16 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
     int B = (int)std::min<size_t>((size_t)nshots, (budget - fixed) / per_slot);
     if (o.batch > 0) B = std::min(B, o.batch);
     {
+        // heights without the tuner (modelling, single wavefields, RTM_B200_TUNE=0): 16 rows for the
+        // velocities and 8 for the pressures; 8 for all, and with that the merged backward launches,
+        // where a batch has fewer than 1.5 million cells and its launches last as long as one tile's
+        // chain (modelling shots of 1801x451, us a step at 8/8, 16/8, 16/16: 1 shot 14.6 15.1 16.1,
+        // 2 23.2 21.5 22.2, 16 137 132 141, 64 523 492 534; migrating 1 shot merged at 8 rows 36.0,
+        // 16/8 44.0, 4 shots 110 and 110).  The other imaging conditions keep 16: see tune_heights.
+        if (!o.extra_images) {
+            ss->bz_pres = ss->bz_pres_recon = 8;
+            if ((double)std::max(B, 1) * big.X * big.Z < 1.5e6) ss->bz_vel = ss->bz_vel_recon = 8;
+        }
         const char *e = std::getenv("RTM_B200_BZ_VEL");
         if (e && *e) ss->bz_vel = std::atoi(e);
         e = std::getenv("RTM_B200_BZ_VEL_RECON");
