@@ -1049,13 +1049,15 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
                 });
     }
     {
-        // a batch whose fields stay in L2 (about 10 arrays per shot): the tiles with PML, source,
+        // batches of up to 400 MB of fields (about 10 arrays per shot): the tiles with PML, source,
         // receiver or strip cells first, since they take two to three times as long as interior
-        // ones and the blocks take tiles as they finish; larger batches keep the tiles in field
-        // order, for the L2 reuse of halo rows between neighbours
+        // ones and would hold up a launch's end; larger batches have many tiles per block and keep
+        // them in field order, for the L2 reuse of halo rows between neighbours.  Shots of 1801x451
+        // (33 MB each), us a step in field order / heavy first: 1 shot 40.2 / 34.8, 4 shots 114 / 103,
+        // 8 202 / 193, 10 240 / 235, 12 279 / 276, 16 355 / 361; 12 shots of 545x395 124 / 99.7
         size_t bytes = 0;
         for (int j = 0; j < n; j++) bytes += (size_t)10 * 4 * ss->shots[k0 + j].pitch * ss->shots[k0 + j].Z;
-        br.heavy_first = bytes <= ((size_t)160 << 20);
+        br.heavy_first = bytes <= ((size_t)400 << 20);
         if (br.heavy_first)
             for (std::vector<TileRef> *v : {&tiles, &tiles_p, &tiles_r, &tiles_pr})
                 std::stable_partition(v->begin(), v->end(), [](const TileRef &t) { return !(t.interior & 1); });
@@ -1637,17 +1639,19 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
 }
 
 // ---- tuner --------------------------------------------------------------------------
-// The split stencil kernels take 8-, 16- or 32-row tiles, and the backward pass runs in four
+// The split stencil kernels take 8-, 16- or 32-row tiles (12-row ones too in the pipelined form), and the backward pass runs in four
 // launches per step or in two merged ones; which is fastest depends on the grid (partial tiles,
 // the share of PML-band and edge tiles), on the shots per launch (tiles to fill 148 SMs) and on
 // the kernel.  Before the first batch of a launch shape, on that batch's own buffers: every
 // height is timed per kernel (two untimed and four timed source-pass and backward steps, no
 // strips saved), which gives each family its fastest one: forward/receiver velocity (one tile
 // list), reconstruction velocity, forward/receiver pressure (one tile list), reconstruction
-// pressure.  Then whole steps are timed back to back for that choice in separate launches and
-// for merged launches at 8 and 16 rows (merging needs one height), and the fastest plan is kept.
+// pressure.  Then whole steps are timed back to back for that choice in separate launches, for the
+// same with the velocity reconstruction at the other velocities' height, and for merged launches
+// at 8 and 16 rows (merging needs one height), and the fastest plan is kept.
 // The batch is set up again afterwards, so the trial steps leave nothing behind; plans do not
-// change the results (tested bit for bit).  Choices are kept per process by launch shape and,
+// change the results (tested bit for bit) but for the forward pressure's interior tiles, whose
+// update fuses one product: which cells those are depends on the height.  Choices are kept per process by launch shape and,
 // with RTM_B200_TUNE_CACHE=<file>, in that file ("key vel vel_recon pres pres_recon plan" lines,
 // plan a bit set: forms of vel, vel_recon, pres, pres_recon, then 16 for merged launches) across
 // processes.  The whole-step kernel's tile height is chosen the same way (tune_step_height).

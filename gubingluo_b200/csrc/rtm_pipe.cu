@@ -29,6 +29,13 @@
 //     copies of what no kernel of the pass writes (1/rho or kappa, damping factors) start before
 //     that wait.
 //
+// What bounds it: 64 shots of 1801x451, us a launch (one tile per block before; each field read and
+// written once at 6.46 TB/s): receiver velocity 192 (248; 191), forward velocity with its strips 210
+// (251 + 28; 193), receiver pressure and imaging 317 (347; 302): the memory's rate.  Forward pressure
+// 258 (281; 187): latency of shared-memory reads and instructions.  Reconstruction 171 and 140 (191,
+// 176; 144, 120): the tiles with strips.  One shot of 401x201: 4.6 us a launch (7 launches of 7 us a
+// step before, 4 now): one tile's chain of copy, sums and stores.
+//
 // Reference kernels these replace: see rtm_stencil.cu.
 #include <atomic>
 #include <type_traits>
@@ -767,7 +774,9 @@ __global__ void __launch_bounds__(Pipe<BZ, PM, VM, ACC, THIN>::threads, Pipe<BZ,
     if (threadIdx.x >= 32 * NC) {   // the producer warp
         // the tile being filled and the one after it: in launches of many tiles per block every
         // step-th tile; in shorter ones, where a block with slow tiles would hold up the launch,
-        // claimed from the counter, one fill ahead of the loads that need it
+        // claimed from the counter, one fill ahead of the loads that need it (one shot of 1801x451:
+        // blocks end after 17 / 22 / 32 us, first / median / last, with a stride and 21.7 / 23.1 / 24.3
+        // claimed; at 64 shots, 100 tiles a block, claiming costs 1-2%)
         const bool dynamic = n <= 16 * step;
         // long lists run backwards in every other launch: what the launch before touched last is
         // still in L2
