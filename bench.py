@@ -199,8 +199,8 @@ def ncu_traffic_per_unit(kernel: str, X: int, Z: int):
 
 # ------------------------------------------------------------------------------------------
 # kernel families timed by the session (split kernels; whole-step kernel)
-KERNEL_FAMILIES = ("vel_fwd", "pres_fwd", "vel_recon", "pres_recon", "vel_recv", "pres_recv", "step_fwd", "step_recon",
-                   "step_recv", "pass_fwd", "pass_bwd")
+KERNEL_FAMILIES = ("vel_fwd", "pres_fwd", "vel_recon", "pres_recon", "vel_recv", "pres_recv", "recon_recv", "recv_recon",
+                   "step_fwd", "step_recon", "step_recv", "pass_fwd", "pass_bwd")
 # the other kernels of a step, timed the same way and reported beside the stencil families
 # (strip_pack runs once per 32 source-pass steps, image_flush once per 32 backward steps)
 AUX_FAMILIES = ("strip_save", "strip_pack", "image_flush")
@@ -216,11 +216,12 @@ def kernel_bytes(kind: str, X: int, Z: int, nxi: int, nzi: int, nrec: int, accum
       vel_recon:  read ps, 1/rho; read+write vxs, vzs on the interior  24 B per interior cell
       pres_recon: read vxs, vzs, kappa; read+write ps on the interior  20 B per interior cell
       pres_recv adds the imaging: read ps, read+write g1 and illum     4 + 4*accum B per interior cell
+      recon_recv, recv_recon (merged backward launches): pres_recon + vel_recv, pres_recv + vel_recon
       step_fwd, step_recv (whole step): read p, vx, vz, 1/rho, kappa; write p, vx, vz   32 B per padded cell
                            + sx, sz read and written in the band       +16 B per band cell
       step_recon: the same on the interior, with both strip sets       32 B per interior cell
-    plus the boundary strips the reconstruction kernels read (the forward strips are written
-    by a separate copy kernel).  pass_fwd / pass_bwd (persistent passes, one launch per pass of
+    plus the boundary strips the reconstruction kernels read (those that the forward kernels write
+    are not counted).  pass_fwd / pass_bwd (persistent passes, one launch per pass of
     nt steps): the per-step kernels' bytes times the steps, with the strip saves."""
     cells, inner = X * Z, nxi * nzi
     band = cells - inner
@@ -237,6 +238,8 @@ def kernel_bytes(kind: str, X: int, Z: int, nxi: int, nzi: int, nrec: int, accum
         "step_recon": 32 * inner + 2 * strips,
         "step_recv": 32 * cells + 16 * band + (4 + 4 * accum_bytes) * inner + 4 * nrec,
     }
+    table["recon_recv"] = table["pres_recon"] + table["vel_recv"]
+    table["recv_recon"] = table["pres_recv"] + table["vel_recon"]
     # persistent passes (one launch per pass): the per-step kernels' bytes times the steps
     table["pass_fwd"] = nt * (table["vel_fwd"] + table["pres_fwd"] + 8 * 40 * (nxi + nzi))
     table["pass_bwd"] = (nt - 1) * (table["vel_recon"] + table["pres_recon"] + table["vel_recv"] + table["pres_recv"])
