@@ -1639,8 +1639,8 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
 }
 
 // ---- tuner --------------------------------------------------------------------------
-// The split stencil kernels take 8-, 16- or 32-row tiles (12-row ones too in the pipelined form), and the backward pass runs in four
-// launches per step or in two merged ones; which is fastest depends on the grid (partial tiles,
+// The split stencil kernels take 8-, 12- or 16-row tiles (the one-column form 8, 16 or 32), and
+// the backward pass runs in four launches per step or in two merged ones; which is fastest depends on the grid (partial tiles,
 // the share of PML-band and edge tiles), on the shots per launch (tiles to fill 148 SMs) and on
 // the kernel.  Before the first batch of a launch shape, on that batch's own buffers: every
 // height is timed per kernel (two untimed and four timed source-pass and backward steps, no
@@ -1771,7 +1771,13 @@ static int tune_heights(rtm_session *ss, int k0, int n)
         }
     }
     if (ss->fused) return tune_step_height(ss, k0, n, key, path);
-    const int nc = ss->vec[0] ? 4 : 3, cand[4] = {8, 16, 32, 12};   // tile heights
+    // tile heights (32 rows leave the pipelined kernels one block per SM and were in no fastest plan:
+    // 4 shots of 4121x1321, where they come nearest, forward velocity 90.5 against 88 us at 16 rows,
+    // receiver pressure 205 against 190; 12 rows pay from 1.5 million cells a batch: one shot of
+    // 1801x451 receiver pressure 12.8 us at 8 rows and 13.8 at 12, 64 shots 360 and 317)
+    double cells = 0;
+    for (int j = 0; j < n; j++) cells += (double)ss->shots[k0 + j].X * ss->shots[k0 + j].Z;
+    const int nc = ss->vec[0] && cells < 1.5e6 ? 2 : 3, cand[3] = {8, 16, ss->vec[0] ? 12 : 32};
     ss->merge = false;
     const char *names[6] = {"vel_fwd", "pres_fwd", "vel_recon", "pres_recon", "vel_recv", "pres_recv"};
     std::vector<std::array<double, 6>> ms(nc, std::array<double, 6>{});
@@ -1835,8 +1841,6 @@ static int tune_heights(rtm_session *ss, int k0, int n)
         // pressure's interior tiles fuse one product (rtm_pipe.cu), so its tile height reaches the
         // last bit of the fields: a fixed height by the batch's cells, 8 rows below 6 million (where
         // 16 leave SMs idle) and 16 above
-        double cells = 0;
-        for (int j = 0; j < n; j++) cells += (double)ss->shots[k0 + j].X * ss->shots[k0 + j].Z;
         best[2] = cells < 6e6 ? 8 : 16;
     }
     const auto use = [&](const std::array<int, 4> &h, bool merge) {

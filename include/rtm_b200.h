@@ -242,8 +242,8 @@ unsigned long long rtm_session_config_hash(rtm_session *ss);
 int rtm_session_guard_count(rtm_session *ss);
 /* Rows per stencil tile in use: forward and receiver velocity, reconstruction velocity,
  * forward and receiver pressure, reconstruction pressure (with the whole-step kernel, its tile
- * height in all four).  Chosen, with the kernel form of each family, per launch shape by timing
- * 8-, 16- and 32-row tiles in both forms before the first batch of that shape
+ * height in all four).  Chosen per launch shape by timing 8-, 12- and 16-row tiles (8, 16, 32
+ * in the one-column form) and merged backward launches before the first batch of that shape
  * (RTM_B200_TUNE=0, or RTM_B200_BZ_VEL / _VEL_RECON / _PRES / _PRES_RECON set, turns that off;
  * RTM_B200_BZ_PRES sets both pressure heights unless _PRES_RECON is given;
  * RTM_B200_KERNELS=scalar|vector fixes the form; choices persist across processes in
