@@ -79,7 +79,10 @@ __global__ void k_narrow(const double *__restrict__ src, float *__restrict__ dst
 }  // namespace
 
 // dst (packed rows of row_bytes) <- rows of the device array src, src_pitch bytes apart, on the
-// current device, whose writers have finished.  narrow: src holds doubles (contiguous), dst floats.
+// current device.  The library's own writers have finished; a caller's work on the array in the
+// default stream or in one that synchronises with it (an all-reduce of the stacked images, whose
+// addresses are public) is waited for as a plain cudaMemcpy waits: the lanes' streams would not.
+// narrow: src holds doubles (contiguous), dst floats.
 int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, size_t rows, bool narrow)
 {
     if (src_pitch == row_bytes || rows == 1) {   // contiguous: rows of a chunk
@@ -100,6 +103,10 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     const size_t per = kChunk / row_bytes, n = (rows + per - 1) / per;   // rows per chunk, chunks
     int dev = 0;
     cudaError_t first = cudaGetDevice(&dev);
+    if (first == cudaSuccess) {
+        char head[4];   // a word through the default stream, behind what is queued there (8 us)
+        first = cudaMemcpy(head, src, sizeof(head), cudaMemcpyDeviceToHost);
+    }
     if (first != cudaSuccess) return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(first));
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
