@@ -352,10 +352,12 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
             ca.out[k] = (double2 *)p.chirp[k];
         }
         const size_t smem = fk::smem_bytes(mt);
-        // (attributes of the instances on this device; setting them again is harmless)
-        CKI(cudaFuncSetAttribute(fk::k_chirps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the kernels' limits on this device, which every plan shares: always those of the longest
+        // transform, since a shorter plan's own sizes would be too low for the plans kept beside it
+        const int limit = (int)fk::smem_bytes(fk::pow2_for(fk::kMaxN));
+        CKI(cudaFuncSetAttribute(fk::k_chirps, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
         for (auto *f : {fk::k_fk_time, fk::k_fk_space, fk::k_fk_filter, fk::k_fk_back})
-            CKI(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CKI(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
         fk::k_twiddles<<<8, 256, 0, st>>>((double2 *)p.tw, mt);
         fk::k_chirps<<<3, 512, smem, st>>>(ca, (const double2 *)p.tw, mt);
         CKI(cudaGetLastError());
