@@ -370,6 +370,17 @@ static int acc_bytes(const rtm_options &o)
     return o.accum_fp64 == RTM_ACC_FP64 || o.accum_fp64 == RTM_ACC_KAHAN ? 8 : 4;
 }
 
+// Tile height of the forward and receiver pressure in a session with the other imaging conditions.
+// It reaches the last bit of the source wavefield there (StepArgs::fuse), so it follows from the session's
+// shots alone, not from the batch, the tuner or what is resumed: 8 rows where all shots together have
+// fewer than 6 million cells (16 leave SMs idle), else 16.
+static int extra_pres_height(const rtm_session *ss)
+{
+    double cells = 0;
+    for (const ShotState &sh : ss->shots) cells += (double)sh.X * sh.Z;
+    return cells < 6e6 ? 8 : 16;
+}
+
 // Tiles of one X x Z shot at the shortest tile height the tuner or the environment may choose.
 static int max_shot_tiles(int X, int Z)
 {
@@ -491,8 +502,11 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
         // where a batch has fewer than 1.5 million cells and its launches last as long as one tile's
         // chain (modelling shots of 1801x451, us a step at 8/8, 16/8, 16/16: 1 shot 14.6 15.1 16.1,
         // 2 23.2 21.5 22.2, 16 137 132 141, 64 523 492 534; migrating 1 shot merged at 8 rows 36.0,
-        // 16/8 44.0, 4 shots 110 and 110).  The other imaging conditions keep 16: see tune_heights.
-        if (!o.extra_images) {
+        // 16/8 44.0, 4 shots 110 and 110).  With the other imaging conditions 16 rows, the
+        // forward and receiver pressure by their own rule
+        if (o.extra_images) {
+            ss->bz_pres = extra_pres_height(ss);
+        } else {
             ss->bz_pres = ss->bz_pres_recon = 8;
             if ((double)std::max(B, 1) * big.X * big.Z < 1.5e6) ss->bz_vel = ss->bz_vel_recon = 8;
         }
@@ -1145,6 +1159,7 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
         a.c10[i] = ss->coef_host[90 + i];
         a.c2[i] = make_float2(a.c10[i], a.c10[i]);
     }
+    a.fuse = o.extra_images != 0;
     a.dt = s.dt;
     a.dtx = s.dt / s.dx;   // rtm_model.cu:73-74
     a.dtz = s.dt / s.dz;
@@ -1650,8 +1665,8 @@ static int batch_backward(rtm_session *ss, BatchRun &br)
 // same with the velocity reconstruction at the other velocities' height, and for merged launches
 // at 8 and 16 rows (merging needs one height), and the fastest plan is kept.
 // The batch is set up again afterwards, so the trial steps leave nothing behind; plans do not
-// change the results (tested bit for bit) but for the forward pressure's interior tiles, whose
-// update fuses one product: which cells those are depends on the height.  Choices are kept per process by launch shape and,
+// change the results (tested bit for bit; with the other imaging conditions the forward and receiver
+// pressure keep one height, extra_pres_height).  Choices are kept per process by launch shape and,
 // with RTM_B200_TUNE_CACHE=<file>, in that file ("key vel vel_recon pres pres_recon plan" lines,
 // plan a bit set: forms of vel, vel_recon, pres, pres_recon, then 16 for merged launches) across
 // processes.  The whole-step kernel's tile height is chosen the same way (tune_step_height).
@@ -1763,7 +1778,7 @@ static int tune_heights(rtm_session *ss, int k0, int n)
             }
             ss->bz_vel = it->second[0];
             ss->bz_vel_recon = it->second[1];
-            ss->bz_pres = it->second[2];
+            ss->bz_pres = ss->o.extra_images ? extra_pres_height(ss) : it->second[2];
             ss->bz_pres_recon = it->second[3];
             for (int f = 0; f < 4; f++) ss->vec[f] = (it->second[4] >> f) & 1;
             ss->merge = (it->second[4] & 16) != 0;
@@ -1836,13 +1851,7 @@ static int tune_heights(rtm_session *ss, int k0, int n)
                                      argmin([&](int c) { return ms[c][2]; }),
                                      argmin([&](int c) { return ms[c][1] + ms[c][5]; }),
                                      argmin([&](int c) { return ms[c][3]; })};
-    if (ss->vec[0] && ss->o.extra_images) {
-        // the wavefield decomposition decides on the signs of products near zero, and the forward
-        // pressure's interior tiles fuse one product (rtm_pipe.cu), so its tile height reaches the
-        // last bit of the fields: a fixed height by the batch's cells, 8 rows below 6 million (where
-        // 16 leave SMs idle) and 16 above
-        best[2] = cells < 6e6 ? 8 : 16;
-    }
+    if (ss->o.extra_images) best[2] = extra_pres_height(ss);
     const auto use = [&](const std::array<int, 4> &h, bool merge) {
         ss->bz_vel = h[0];
         ss->bz_vel_recon = h[1];

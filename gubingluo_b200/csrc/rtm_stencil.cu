@@ -395,17 +395,21 @@ __device__ __forceinline__ void pres_tile(const StepArgs &a, int record, const T
             if (MODE == 0) dx_pairs<U, -1, 0>(&colx[(z - z0) * WW], dxs, [&](int j) { return a.c10[j]; });
             if constexpr (MODE == 0 && U == 2) {
                 // the update of both rows in packed pairs as well: per lane the products and the
-                // separately rounded sum and difference of p_interior, so the same bits
+                // separately rounded sum and difference of p_interior, so the same bits.  (Written as
+                // multiply-adds by -1, which round as the sum and the difference do: the assembler
+                // contracts a packed product into a packed addition that follows it.)
                 float dz2[2];
 #pragma unroll
                 for (int u = 0; u < 2; u++)
                     dz2[u] = tap_sum([&](int j) { return a.c10[j]; }, [&](int i) { return q[u + 9 + i]; },
                                      [&](int i) { return q[u + 10 - i]; });
                 const float2 kk = make_float2(ckk[0], ckk[1]);
-                const float2 dxs2 = __fmul2_rn(__fmul2_rn(make_float2(dxs[0], dxs[1]), make_float2(a.dtx, a.dtx)), kk);
-                const float2 dzs2 = __fmul2_rn(__fmul2_rn(make_float2(dz2[0], dz2[1]), make_float2(a.dtz, a.dtz)), kk);
-                const float2 sum = __fadd2_rn(dxs2, dzs2);
-                const float2 pn = __fadd2_rn(make_float2(cp0[0], cp0[1]), make_float2(-sum.x, -sum.y));
+                const float2 ax = __fmul2_rn(make_float2(dxs[0], dxs[1]), make_float2(a.dtx, a.dtx));
+                const float2 mdzs2 = __fmul2_rn(__fmul2_rn(make_float2(dz2[0], dz2[1]), make_float2(-a.dtz, -a.dtz)), kk);
+                const float2 m1 = make_float2(-1.f, -1.f);
+                const float2 sum = a.fuse ? __ffma2_rn(ax, kk, make_float2(-mdzs2.x, -mdzs2.y))
+                                          : __ffma2_rn(mdzs2, m1, __fmul2_rn(ax, kk));
+                const float2 pn = __ffma2_rn(sum, m1, make_float2(cp0[0], cp0[1]));
                 pp[id0] = pn.x;
                 pp[id0 + pitch] = pn.y;
             } else {

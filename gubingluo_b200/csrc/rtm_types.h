@@ -195,6 +195,12 @@ struct StepArgs {
     int list;
     unsigned *queue;        // two tile counters of the pipelined kernels: a launch takes tiles from
     int qsel;               // queue[qsel] and clears the other one for the launch after it
+    // 1 (sessions with the other imaging conditions): the source pass's interior tiles round p - fma(dt/dx
+    // Dx, kappa, dt/dz Dz kappa) where every other cell rounds both products.  Those conditions switch on the
+    // signs of products near zero, so a last bit of p changes their images by whole terms; the
+    // rounding and the tile height (extra_pres_height) are kept as they were, so that images of
+    // earlier surveys come out the same
+    int fuse;
     int save;               // 1: the pipelined source-pass kernels save their tiles' strip cells
     int prefetch;           // 1: the stencil kernels prefetch their tile's operand rows into L2
 };
