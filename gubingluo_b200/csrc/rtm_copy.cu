@@ -103,11 +103,13 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     const size_t per = kChunk / row_bytes, n = (rows + per - 1) / per;   // rows per chunk, chunks
     int dev = 0;
     cudaError_t first = cudaGetDevice(&dev);
-    if (first == cudaSuccess) {
-        char head[4];   // a word through the default stream, behind what is queued there (8 us)
-        first = cudaMemcpy(head, src, sizeof(head), cudaMemcpyDeviceToHost);
+    cudaEvent_t before = nullptr;   // the default stream's work so far, which the lanes wait for
+    if (first == cudaSuccess) first = cudaEventCreateWithFlags(&before, cudaEventDisableTiming);
+    if (first == cudaSuccess) first = cudaEventRecord(before, cudaStreamLegacy);
+    if (first != cudaSuccess) {
+        if (before) cudaEventDestroy(before);
+        return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(first));
     }
-    if (first != cudaSuccess) return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(first));
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
     const int nt = (int)std::min<size_t>(kLanes, n);
@@ -116,6 +118,7 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
         Lane l;
         cudaError_t e = cudaSetDevice(dev);
         if (e == cudaSuccess && !take(dev, l)) e = cudaErrorMemoryAllocation;
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(l.st, before, 0);
         while (e == cudaSuccess) {
             const size_t c = next.fetch_add(1);
             if (c >= n) break;
@@ -138,6 +141,7 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
         }
         if (e != cudaSuccess) err.store((int)e);
     }
+    cudaEventDestroy(before);
     if (err.load() != (int)cudaSuccess)
         return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString((cudaError_t)err.load()));
     return RTM_OK;
