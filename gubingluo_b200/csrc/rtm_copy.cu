@@ -76,6 +76,19 @@ __global__ void k_narrow(const double *__restrict__ src, float *__restrict__ dst
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = (float)src[i];
 }
 
+// The narrowing copy without a lane: n doubles through a buffer on the stack.
+cudaError_t plain_narrow(float *dst, const double *src, size_t n)
+{
+    double part[4096];
+    for (size_t i = 0; i < n; i += 4096) {
+        const size_t m = std::min<size_t>(4096, n - i);
+        cudaError_t e = cudaMemcpy(part, src + i, m * sizeof(double), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return e;
+        for (size_t k = 0; k < m; k++) dst[i + k] = (float)part[k];
+    }
+    return cudaSuccess;
+}
+
 }  // namespace
 
 // dst (packed rows of row_bytes) <- rows of the device array src, src_pitch bytes apart, on the
@@ -102,24 +115,22 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     }
     const size_t per = kChunk / row_bytes, n = (rows + per - 1) / per;   // rows per chunk, chunks
     int dev = 0;
-    cudaError_t first = cudaGetDevice(&dev);
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(e));
     cudaEvent_t before = nullptr;   // the default stream's work so far, which the lanes wait for
-    if (first == cudaSuccess) first = cudaEventCreateWithFlags(&before, cudaEventDisableTiming);
-    if (first == cudaSuccess) first = cudaEventRecord(before, cudaStreamLegacy);
-    if (first != cudaSuccess) {
-        if (before) cudaEventDestroy(before);
-        return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(first));
-    }
+    bool lanes = cudaEventCreateWithFlags(&before, cudaEventDisableTiming) == cudaSuccess;
+    lanes = lanes && cudaEventRecord(before, cudaStreamLegacy) == cudaSuccess;
+    if (!lanes) cudaGetLastError();
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
-    const int nt = (int)std::min<size_t>(kLanes, n);
+    const int nt = lanes ? (int)std::min<size_t>(kLanes, n) : 1;
 #pragma omp parallel num_threads(nt)
     {
         Lane l;
         cudaError_t e = cudaSetDevice(dev);
-        if (e == cudaSuccess && !take(dev, l)) e = cudaErrorMemoryAllocation;
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(l.st, before, 0);
-        while (e == cudaSuccess) {
+        const bool lane = lanes && e == cudaSuccess && take(dev, l);   // without one this thread copies nothing
+        if (lane) e = cudaStreamWaitEvent(l.st, before, 0);
+        while (lane && e == cudaSuccess) {
             const size_t c = next.fetch_add(1);
             if (c >= n) break;
             const size_t r0 = c * per, nr = std::min(per, rows - r0), bytes = nr * row_bytes;
@@ -141,9 +152,18 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
         }
         if (e != cudaSuccess) err.store((int)e);
     }
-    cudaEventDestroy(before);
-    if (err.load() != (int)cudaSuccess)
-        return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString((cudaError_t)err.load()));
+    if (before) cudaEventDestroy(before);
+    e = (cudaError_t)err.load();
+    const size_t r0 = std::min(next.load() * per, rows);
+    if (e == cudaSuccess && r0 < rows) {
+        // what no lane took (no page-locked memory, stream or event to be had): plain copies
+        void *to = (char *)dst + r0 * row_bytes;
+        const void *from = (const char *)src + r0 * src_pitch;
+        if (narrow) e = plain_narrow((float *)to, (const double *)src + r0 / 4, (rows - r0) / 4);
+        else if (row_bytes == 1) e = cudaMemcpy(to, from, rows - r0, cudaMemcpyDeviceToHost);
+        else e = cudaMemcpy2D(to, row_bytes, from, src_pitch, row_bytes, rows - r0, cudaMemcpyDeviceToHost);
+    }
+    if (e != cudaSuccess) return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(e));
     return RTM_OK;
 }
 
