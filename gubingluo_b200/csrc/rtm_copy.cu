@@ -14,7 +14,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <vector>
 
 #include "rtm_internal.h"
 
@@ -23,15 +22,19 @@ namespace rtm {
 namespace {
 
 constexpr size_t kChunk = (size_t)1 << 20;   // bytes of a lane's page-locked buffer
-constexpr int kLanes = 4;                    // lanes kept by the process (4 MB page-locked at most)
+constexpr int kLanes = 4;                    // lanes of a copy, and those kept per device (4 MB page-locked)
+constexpr int kMaxDevices = 64;              // (lanes of devices beyond are not kept)
 
 struct Lane {
     void *buf = nullptr;
     cudaStream_t st = nullptr;
     int dev = -1;
 };
+// Lanes not in use, per device: lanes of one device must not take the places of another's, whose every
+// copy would then allocate and free its own.
 std::mutex g_mu;
-std::vector<Lane> g_free;   // lanes not in use, at most kLanes
+Lane g_free[kMaxDevices][kLanes];
+int g_kept[kMaxDevices];
 
 void drop(Lane &l)
 {
@@ -43,12 +46,10 @@ bool take(int dev, Lane &l)
 {
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        for (size_t i = 0; i < g_free.size(); i++)
-            if (g_free[i].dev == dev) {
-                l = g_free[i];
-                g_free.erase(g_free.begin() + i);
-                return true;
-            }
+        if (dev < kMaxDevices && g_kept[dev] > 0) {
+            l = g_free[dev][--g_kept[dev]];
+            return true;
+        }
     }
     l.dev = dev;
     if (cudaHostAlloc(&l.buf, kChunk, cudaHostAllocDefault) != cudaSuccess ||
@@ -63,8 +64,8 @@ void give(Lane &l)
 {
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if ((int)g_free.size() < kLanes) {
-            g_free.push_back(l);
+        if (l.dev < kMaxDevices && g_kept[l.dev] < kLanes) {
+            g_free[l.dev][g_kept[l.dev]++] = l;
             return;
         }
     }

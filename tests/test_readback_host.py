@@ -4,6 +4,7 @@ import ctypes as C
 import os
 import shutil
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -233,3 +234,29 @@ def test_copies_without_page_locked_memory_or_streams(rb, what, left):
     for seed in range(3):
         _copies(rb, seed)
     assert _var(rb, "stale").value == 0
+
+
+def test_each_device_keeps_its_own_lanes(rb):
+    for d in (0, 1, 2, 0, 1, 2):
+        rb.use_device(d)
+        _copies(rb, d)
+    assert _var(rb, "allocs").value == _var(rb, "live").value <= 3 * 4   # none was freed again
+
+
+def test_copies_of_several_threads_leave_at_most_four_lanes(rb):
+    errors = []
+
+    def work(k):
+        try:
+            for _ in range(4):
+                _copies(rb, k)
+        except BaseException as e:   # (a thread's failure must reach the test)
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert _var(rb, "live").value <= 4 and _var(rb, "stale").value == 0
