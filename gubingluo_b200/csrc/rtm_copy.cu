@@ -7,6 +7,7 @@
 // move chunks through a page-locked buffer and stream of their own, so copies, page faults and
 // host writes overlap, and fp64 images are narrowed by a kernel that writes the page-locked
 // buffer (half the bytes over the bus).  Measured: 1.1 ms and 7 ms.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +30,7 @@ struct Lane {
     void *buf = nullptr;
     cudaStream_t st = nullptr;
     int dev = -1;
+    unsigned long long ctx = 0;   // the context they were made in
 };
 // Lanes not in use, per device: lanes of one device must not take the places of another's, whose every
 // copy would then allocate and free its own.
@@ -42,16 +44,35 @@ void drop(Lane &l)
     if (l.buf) cudaFreeHost(l.buf);
     l = Lane();
 }
-bool take(int dev, Lane &l)
+// Number of the current context, different for every context that the process ever makes (0 where the driver
+// has no such call): a cudaDeviceReset takes the kept lanes' buffers and streams with it, and the
+// device's next context has another number.
+unsigned long long context_id()
+{
+    typedef CUresult (*Fn)(CUcontext, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (Fn)p;
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+bool take(int dev, unsigned long long ctx, Lane &l)
 {
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (dev < kMaxDevices && g_kept[dev] > 0) {
+        while (dev < kMaxDevices && g_kept[dev] > 0) {
             l = g_free[dev][--g_kept[dev]];
-            return true;
+            if (l.ctx == ctx) return true;
+            l = Lane();   // gone with its context
         }
     }
     l.dev = dev;
+    l.ctx = ctx;
     if (cudaHostAlloc(&l.buf, kChunk, cudaHostAllocDefault) != cudaSuccess ||
         cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError();
@@ -124,12 +145,13 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     if (!lanes) cudaGetLastError();
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
+    const unsigned long long ctx = context_id();   // (the library runs in the device's primary context only)
     const int nt = lanes ? (int)std::min<size_t>(kLanes, n) : 1;
 #pragma omp parallel num_threads(nt)
     {
         Lane l;
         cudaError_t e = cudaSetDevice(dev);
-        const bool lane = lanes && e == cudaSuccess && take(dev, l);   // without one this thread copies nothing
+        const bool lane = lanes && e == cudaSuccess && take(dev, ctx, l);   // without one this thread copies nothing
         if (lane) e = cudaStreamWaitEvent(l.st, before, 0);
         while (lane && e == cudaSuccess) {
             const size_t c = next.fetch_add(1);

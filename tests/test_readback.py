@@ -51,3 +51,39 @@ def test_images_wait_for_work_on_the_default_stream(rtmlib, nx, nz, accum, block
         got = ss.images()["image1"].ravel()
         torch.cuda.synchronize()
         assert np.array_equal(got, want.astype(np.float32))
+
+
+RESET = """
+import ctypes as C
+import numpy as np
+import gubingluo_b200 as G
+
+def context():
+    f, q, n = C.c_void_p(), C.c_int(), C.c_ulonglong()
+    assert rt.cudaGetDriverEntryPoint(b"cuCtxGetId", C.byref(f), C.c_ulonglong(0), C.byref(q)) == 0
+    assert C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p)(f.value)(None, C.addressof(n)) == 0
+    return n.value
+
+G.lib()
+rt = C.CDLL("libcudart.so.12")
+obs = np.random.default_rng(0).standard_normal((400, 200)).astype(np.float32)
+a = G.interp_gather(obs, 399, 400, 1e-3, 1e-3)   # 638 KB: through the kept buffers
+before = context()
+assert rt.cudaDeviceReset() == 0
+assert rt.cudaSetDevice(0) == 0 and rt.cudaFree(None) == 0
+assert context() != before, "a new context must have a new number: stopping before the next copy"
+assert np.array_equal(G.interp_gather(obs, 399, 400, 1e-3, 1e-3), a)
+print("same")
+"""
+
+
+@pytest.mark.gpu
+def test_results_after_a_device_reset(rtmlib):
+    """In a process of its own: cudaDeviceReset ends the process's context."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", RESET], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr

@@ -260,3 +260,10 @@ def test_copies_of_several_threads_leave_at_most_four_lanes(rb):
         t.join()
     assert not errors, errors
     assert _var(rb, "live").value <= 4 and _var(rb, "stale").value == 0
+
+
+def test_lanes_lost_in_a_device_reset_are_not_used_again(rb):
+    _copies(rb)
+    rb.reset_device()
+    _copies(rb, 1)
+    assert _var(rb, "stale").value == 0
