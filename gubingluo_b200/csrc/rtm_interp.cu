@@ -276,11 +276,12 @@ int interp_shape(int nx0, int nt0, int nx, int nt, InterpShape &sh)
 }
 
 // Device workspace and cuFFT plans for one interpolation shape (kept while the shape repeats);
-// with_out: room for the result too (p.d_out).
+// with_out: room for the result too (p.d_out), which a plan made without it has not.
 static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool with_out)
 {
     const bool own = sh.fk && own_transforms(sh);
-    if (p.work && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (!sh.fk || own || p.plans)) {
+    if (p.work && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (!sh.fk || own || p.plans) &&
+        (p.d_out || !with_out)) {
         if (p.plans) {
             CKF(cufftSetStream((cufftHandle)p.p_k, st));
             CKF(cufftSetStream((cufftHandle)p.p_s, st));

@@ -1,4 +1,7 @@
 """Kept workspaces of the gather resampling (rtm_interp.cu) beside other shapes and callers."""
+import os
+import shutil
+import subprocess
 import threading
 
 import numpy as np
@@ -63,3 +66,88 @@ def test_plans_of_two_lengths_in_two_threads(rtmlib):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+# calls of the library's own C++ entry to the resampling, which Python does not reach: argv[1] names
+# the check, and the result of a fresh plan is what every other call must give
+OWN_ENTRY = r"""
+#include <cuda_runtime.h>
+#include <dlfcn.h>
+
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "rtm_internal.h"
+
+static int fail_next = 0;
+extern "C" cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v)   // before the runtime's
+{
+    typedef cudaError_t (*Fn)(const void *, cudaFuncAttribute, int);
+    if (fail_next) {
+        fail_next--;
+        return cudaErrorInvalidValue;
+    }
+    return ((Fn)dlsym(RTLD_NEXT, "cudaFuncSetAttribute"))(f, a, v);
+}
+
+int main(int, char **argv)
+{
+    const std::string what = argv[1];
+    const int nx0 = 41, nt0 = 1500, nx = 81, nt = 1500;
+    const float dt = 1e-3f;
+    const size_t n = (size_t)nt * nx;
+    std::vector<float> in((size_t)nx0 * nt0), want(n), got(n);
+    for (size_t i = 0; i < in.size(); i++) in[i] = (float)((i * 2654435761u >> 8) % 1000) / 1000.0f - 0.5f;
+    cudaStream_t st;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) return 2;
+    float *out;
+    if (cudaMalloc(&out, 4 * n)) return 2;
+    rtm::InterpPlan fresh, p;
+    const auto run = [&](rtm::InterpPlan &q, float *to) {
+        return rtm::interp_gather_device(q, in.data(), nx0, nt0, to, nx, nt, dt, dt, 0, st, nullptr);
+    };
+    const auto read = [&](std::vector<float> &v, const float *from) {
+        return cudaMemcpyAsync(v.data(), from, 4 * n, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+               cudaStreamSynchronize(st) == cudaSuccess;
+    };
+    if (run(fresh, out) || !read(want, out)) return 2;
+    const float *from = out;
+    if (what == "own result") {   // a plan made for a caller's buffer, then asked for one of its own
+        if (run(p, out)) return 3;
+        if (run(p, nullptr)) return 4;
+        from = p.d_out;
+        if (!from) return 5;
+    } else if (what == "interrupted") {   // a plan that failed half way, then asked again
+        fail_next = 1;
+        if (!run(p, out)) return 3;
+        if (run(p, out)) return 4;
+    }
+    if (!read(got, from)) return 6;
+    p.release();
+    fresh.release();
+    std::puts(std::memcmp(got.data(), want.data(), 4 * n) ? "different" : "same");
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def own_entry(rtmlib, tmp_path_factory):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    lib = os.path.join(root, "gubingluo_b200")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")))
+    d = tmp_path_factory.mktemp("own_entry")
+    (d / "own.cpp").write_text(OWN_ENTRY)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-rdynamic", "-I" + os.path.join(root, "include"),
+                    "-I" + os.path.join(lib, "csrc"), "-I" + cuda + "/include", "-o", str(d / "own"), str(d / "own.cpp"),
+                    os.path.join(lib, "librtm_b200.so"), "-L" + cuda + "/lib64", "-lcudart", "-ldl",
+                    "-Wl,-rpath," + lib, "-Wl,-rpath," + cuda + "/lib64"], check=True)
+    return str(d / "own")
+
+
+@pytest.mark.gpu
+def test_a_plan_without_room_for_the_result_is_not_asked_for_it(own_entry):
+    r = subprocess.run([own_entry, "own result"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "same", (r.returncode, r.stderr)
