@@ -56,6 +56,7 @@ int interp_shape(int nx0, int nt0, int nx, int nt, InterpShape &sh);
 // shape repeats (shots of a survey usually share it).
 struct InterpPlan {
     InterpShape shape{};
+    bool ready = false;                   // everything below was made (a plan that failed half way is not)
     void *work = nullptr;                 // one allocation holding everything below
     float *d_in = nullptr, *d_tmp = nullptr, *d_out = nullptr;
     void *K = nullptr, *S = nullptr, *Z = nullptr, *G1 = nullptr, *G = nullptr;   // double2 arrays

@@ -280,8 +280,7 @@ int interp_shape(int nx0, int nt0, int nx, int nt, InterpShape &sh)
 static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool with_out)
 {
     const bool own = sh.fk && own_transforms(sh);
-    if (p.work && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (!sh.fk || own || p.plans) &&
-        (p.d_out || !with_out)) {
+    if (p.ready && std::memcmp(&p.shape, &sh, sizeof(sh)) == 0 && (p.d_out || !with_out)) {
         if (p.plans) {
             CKF(cufftSetStream((cufftHandle)p.p_k, st));
             CKF(cufftSetStream((cufftHandle)p.p_s, st));
@@ -394,6 +393,7 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
         CKF(cufftSetStream((cufftHandle)p.p_x, st));
         CKF(cufftSetStream((cufftHandle)p.p_t, st));
     }
+    p.ready = true;
     return RTM_OK;
 }
 

@@ -151,3 +151,9 @@ def own_entry(rtmlib, tmp_path_factory):
 def test_a_plan_without_room_for_the_result_is_not_asked_for_it(own_entry):
     r = subprocess.run([own_entry, "own result"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "same", (r.returncode, r.stderr)
+
+
+@pytest.mark.gpu
+def test_a_plan_that_failed_half_way_is_made_again(own_entry):
+    r = subprocess.run([own_entry, "interrupted"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "same", (r.returncode, r.stderr)
