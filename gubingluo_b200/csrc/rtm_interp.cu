@@ -330,7 +330,11 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
         o_G = take(sizeof(double2) * (size_t)sh.nx * sh.nt0);
         o_zm = take(sizeof(unsigned));
     }
-    CKI(cudaMalloc(&p.work, off));
+    if (cudaMalloc(&p.work, off) != cudaSuccess) {
+        cudaGetLastError();   // (a refusal, not an error of the launches to come)
+        p.work = nullptr;
+        return fail(RTM_ERR_NOMEM, "resampling: device allocation of " + std::to_string(off) + " bytes failed");
+    }
     char *b = (char *)p.work;
     for (const auto &g : p.guards) CKI(cudaMemsetAsync(b + g.first, 0xA5, g.second, st));
     p.d_in = (float *)(b + o_in);

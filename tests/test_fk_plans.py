@@ -157,3 +157,18 @@ def test_a_plan_without_room_for_the_result_is_not_asked_for_it(own_entry):
 def test_a_plan_that_failed_half_way_is_made_again(own_entry):
     r = subprocess.run([own_entry, "interrupted"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "same", (r.returncode, r.stderr)
+
+
+# a result of 200 GB: refused with the code for memory, and the next call is as if nothing had been
+@pytest.mark.gpu
+def test_a_result_beyond_the_device_memory_is_refused(rtmlib):
+    import ctypes as C
+
+    G = rtmlib
+    obs = _record(10, 25, 0)
+    want = G.interp_gather(obs, 49, 20, 1e-3, 2e-3)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    out = np.zeros(25, np.float32)   # (never written: the call fails before)
+    rc = G.lib().rtm_interp_gather(p(obs), 25, 10, p(out), 25, 2_000_000_000, 1e-3, 2e-3, 0, 0)
+    assert rc == -4 and b"alloc" in G.lib().rtm_last_error()
+    assert np.array_equal(G.interp_gather(obs, 49, 20, 1e-3, 2e-3), want)
