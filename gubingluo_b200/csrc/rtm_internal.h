@@ -60,7 +60,7 @@ struct InterpPlan {
     void *work = nullptr;                 // one allocation holding everything below
     float *d_in = nullptr, *d_tmp = nullptr, *d_out = nullptr;
     void *K = nullptr, *S = nullptr, *Z = nullptr, *G1 = nullptr, *G = nullptr;   // double2 arrays
-    void *A = nullptr, *tw = nullptr, *chirp[3] = {nullptr, nullptr, nullptr};   // rtm_fk.cuh's tables
+    void *A = nullptr, *tw = nullptr, *chirp[3] = {}, *phase[3] = {};   // rtm_fk.cuh's tables
     int mt = 0;
     unsigned *zmax = nullptr;
     int p_k = 0, p_s = 0, p_x = 0, p_t = 0;   // cufftHandle values, valid when `plans`

@@ -306,20 +306,22 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
     const size_t o_in = take(sizeof(float) * (size_t)sh.nt0 * sh.nx0);
     const size_t o_out = with_out ? take(sizeof(float) * (size_t)sh.nt * sh.nx) : 0;
     size_t o_tmp = 0, o_K = 0, o_S = 0, o_Z = 0, o_G1 = 0, o_G = 0, o_zm = 0;
-    size_t o_A = 0, o_tw = 0, o_c[3] = {0, 0, 0};
-    const int len[3] = {sh.nt0, sh.nx0, sh.Nx};
+    size_t o_A = 0, o_tw = 0, o_c[3] = {0, 0, 0}, o_p[3] = {0, 0, 0};
+    const int len[3] = {sh.nt0, sh.nx0, sh.Nx}, parts[3] = {sh.lx, sh.lx, 1};
     int mt = 16;
     if (own) {
-        const size_t nh = sh.Nt / 2 + 1;
         for (int l : len) mt = std::max(mt, fk::pow2_for(l));
         o_tmp = take(sizeof(float) * (size_t)sh.nt0 * sh.nx);
-        o_A = take(sizeof(double2) * nh * sh.nx0);
+        o_A = take(sizeof(double2) * (size_t)sh.Nt * ((sh.nx0 + 1) / 2));
         o_K = take(sizeof(double2) * (size_t)sh.nf * sh.nx0);
         o_S = take(sizeof(double2) * (size_t)sh.nf * sh.Nx);
         o_Z = take(sizeof(double2) * (size_t)sh.nf * sh.nx0);
         o_G = take(sizeof(double2) * (size_t)sh.nf * sh.nx);
         o_tw = take(sizeof(double2) * (mt / 4));
-        for (int k = 0; k < 3; k++) o_c[k] = take(sizeof(double2) * fk::pow2_for(len[k]));
+        for (int k = 0; k < 3; k++) {
+            o_c[k] = take(sizeof(double2) * fk::pow2_for(len[k]));
+            o_p[k] = take(sizeof(double2) * (size_t)parts[k] * len[k]);
+        }
         o_zm = take(sizeof(unsigned));
     } else if (sh.fk) {
         o_tmp = take(sizeof(float) * (size_t)sh.nt0 * sh.nx);
@@ -350,8 +352,13 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
         p.zmax = (unsigned *)(b + o_zm);
         p.mt = mt;
         fk::ChirpArgs ca;
+        fk::PhaseArgs pa;
         for (int k = 0; k < 3; k++) {
             p.chirp[k] = b + o_c[k];
+            p.phase[k] = b + o_p[k];
+            pa.len[k] = len[k];
+            pa.parts[k] = parts[k];
+            pa.out[k] = (double2 *)p.phase[k];
             ca.len[k] = len[k];
             ca.out[k] = (double2 *)p.chirp[k];
         }
@@ -363,6 +370,7 @@ static int plan_for(InterpPlan &p, const InterpShape &sh, cudaStream_t st, bool 
         for (auto *f : {fk::k_fk_time, fk::k_fk_space, fk::k_fk_filter, fk::k_fk_back})
             CKI(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
         fk::k_twiddles<<<8, 256, 0, st>>>((double2 *)p.tw, mt);
+        fk::k_phases<<<dim3(32, 3), 256, 0, st>>>(pa);
         fk::k_chirps<<<3, 512, smem, st>>>(ca, (const double2 *)p.tw, mt);
         CKI(cudaGetLastError());
     } else if (sh.fk) {
@@ -422,17 +430,16 @@ static int interp_run(InterpPlan &p, float *out, float dt, float dt0, int mirror
         a.A = (double2 *)p.A; a.K = (double2 *)p.K; a.S = (double2 *)p.S; a.Z = (double2 *)p.Z; a.G = (double2 *)p.G;
         a.zmax = p.zmax;
         a.ct = (const double2 *)p.chirp[0]; a.cx = (const double2 *)p.chirp[1]; a.cX = (const double2 *)p.chirp[2];
+        a.pt = (const double2 *)p.phase[0]; a.px = (const double2 *)p.phase[1]; a.pX = (const double2 *)p.phase[2];
         a.tw = (const double2 *)p.tw;
         a.mt = p.mt;
         a.out = sh.sinc ? p.d_tmp : out;
         CKI(cudaMemsetAsync(p.zmax, 0, sizeof(unsigned), st));
         const int mT = fk::pow2_for(sh.nt0), mx = fk::pow2_for(sh.nx0), mX = fk::pow2_for(sh.Nx);
-        // threads: one radix-4 butterfly each per stage up to 512 (warps are whole)
-        const auto threads = [](int m) { return std::min(512, std::max(32, m / 4)); };
-        fk::k_fk_time<<<dim3(sh.nx0, sh.lx), threads(mT), fk::smem_bytes(mT), st>>>(a);
-        fk::k_fk_space<<<a.nh, threads(mx), fk::smem_bytes(mx), st>>>(a);
-        fk::k_fk_filter<<<sh.nf, threads(mX), fk::smem_bytes(mX), st>>>(a);
-        fk::k_fk_back<<<sh.nx, threads(mT), fk::smem_bytes(mT), st>>>(a);
+        fk::k_fk_time<<<dim3((sh.nx0 + 1) / 2, sh.lx), fk::threads(mT), fk::smem_bytes(mT), st>>>(a);
+        fk::k_fk_space<<<dim3(a.nh, sh.lx + 1), fk::threads(mx), fk::smem_bytes(mx), st>>>(a);
+        fk::k_fk_filter<<<sh.nf, fk::threads(mX), fk::smem_bytes(mX), st>>>(a);
+        fk::k_fk_back<<<(sh.nx + 1) / 2, fk::threads(mT), fk::smem_bytes(mT), st>>>(a);
         if (launches) *launches += 4;
         src = p.d_tmp;
         ld = sh.nx;

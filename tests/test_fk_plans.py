@@ -172,3 +172,20 @@ def test_a_result_beyond_the_device_memory_is_refused(rtmlib):
     rc = G.lib().rtm_interp_gather(p(obs), 25, 10, p(out), 25, 2_000_000_000, 1e-3, 2e-3, 0, 0)
     assert rc == -4 and b"alloc" in G.lib().rtm_last_error()
     assert np.array_equal(G.interp_gather(obs, 49, 20, 1e-3, 2e-3), want)
+
+
+# odd and even counts of traces in and out (two share a transform in time), a pair whose traces differ by
+# 1e5 in size, and lengths in x whose power of two (16 to 8192 points) takes every order of passes
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx0,nt0,lx", [(2, 9, 2), (3, 40, 2), (4, 41, 3), (5, 8, 4), (17, 30, 3), (33, 60, 5),
+                                        (65, 130, 2), (129, 20, 3), (250, 30, 4), (512, 21, 4), (1300, 12, 3)])
+@pytest.mark.parametrize("mirror", [0, 1])
+def test_pairs_of_traces_and_every_order_of_passes(rtmlib, nx0, nt0, lx, mirror):
+    from test_fk import _fk
+
+    obs = _record(nt0, nx0, nx0 * lx) * np.where(np.arange(nx0) % 4 == 1, 1e-5, 1.0).astype(np.float32)
+    nx = lx * (nx0 - 1) + 1
+    got = rtmlib.interp_gather(obs, nx, nt0, 1e-3, 1e-3, mirror)
+    want = _fk(obs, nx, lx, mirror)
+    # as test_fk: float32 rounding of the result and of max|Z|
+    assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
