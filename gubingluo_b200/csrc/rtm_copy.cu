@@ -114,10 +114,8 @@ cudaError_t plain_narrow(float *dst, const double *src, size_t n)
 }  // namespace
 
 // dst (packed rows of row_bytes) <- rows of the device array src, src_pitch bytes apart, on the
-// current device.  The library's own writers have finished; a caller's work on the array in the
-// default stream or in one that synchronises with it (an all-reduce of the stacked images, whose
-// addresses are public) is waited for as a plain cudaMemcpy waits: the lanes' streams would not.
-// narrow: src holds doubles (contiguous), dst floats.
+// current device, whose writers have finished: unlike a plain cudaMemcpy, the lanes' streams do not wait for
+// the default stream.  narrow: src holds doubles (contiguous), dst floats.
 int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, size_t rows, bool narrow)
 {
     if (src_pitch == row_bytes || rows == 1) {   // contiguous: rows of a chunk
@@ -139,20 +137,15 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail(RTM_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(e));
-    cudaEvent_t before = nullptr;   // the default stream's work so far, which the lanes wait for
-    bool lanes = cudaEventCreateWithFlags(&before, cudaEventDisableTiming) == cudaSuccess;
-    lanes = lanes && cudaEventRecord(before, cudaStreamLegacy) == cudaSuccess;
-    if (!lanes) cudaGetLastError();
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
     const unsigned long long ctx = context_id();   // (the library runs in the device's primary context only)
-    const int nt = lanes ? (int)std::min<size_t>(kLanes, n) : 1;
+    const int nt = (int)std::min<size_t>(kLanes, n);
 #pragma omp parallel num_threads(nt)
     {
         Lane l;
         cudaError_t e = cudaSetDevice(dev);
-        const bool lane = lanes && e == cudaSuccess && take(dev, ctx, l);   // without one this thread copies nothing
-        if (lane) e = cudaStreamWaitEvent(l.st, before, 0);
+        const bool lane = e == cudaSuccess && take(dev, ctx, l);   // without one this thread copies nothing
         while (lane && e == cudaSuccess) {
             const size_t c = next.fetch_add(1);
             if (c >= n) break;
@@ -175,11 +168,10 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
         }
         if (e != cudaSuccess) err.store((int)e);
     }
-    if (before) cudaEventDestroy(before);
     e = (cudaError_t)err.load();
     const size_t r0 = std::min(next.load() * per, rows);
     if (e == cudaSuccess && r0 < rows) {
-        // what no lane took (no page-locked memory, stream or event to be had): plain copies
+        // what no lane took (no page-locked memory or stream to be had): plain copies
         void *to = (char *)dst + r0 * row_bytes;
         const void *from = (const char *)src + r0 * src_pitch;
         if (narrow) e = plain_narrow((float *)to, (const double *)src + r0 / 4, (rows - r0) / 4);

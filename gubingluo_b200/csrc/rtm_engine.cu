@@ -2219,6 +2219,20 @@ int rtm_session_nrec(rtm_session *ss, int k)
     return ss->shots[k].g.nrec;
 }
 
+// Before the stacked images are read: their addresses are public (rtm_session_image_ptrs), so a caller's work
+// on them may be queued in the default stream, or in one that synchronises with it.  A plain copy of the
+// images would wait for it; the streams of copy_out do not.
+static int wait_for_callers_work(rtm_session *ss)
+{
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ev, cudaStreamLegacy);
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev);
+    cudaEventDestroy(ev);
+    CK(e);
+    return RTM_OK;
+}
+
 static int copy_image(rtm_session *ss, void *dev, float *out)
 {
     if (!out) return RTM_OK;
@@ -2232,6 +2246,7 @@ int rtm_session_get_images(rtm_session *ss, float *image1, float *image2s, float
     CK(cudaSetDevice(ss->dev));
     CK(cudaStreamSynchronize(ss->stream));
     int rc;
+    if ((rc = wait_for_callers_work(ss))) return rc;
     if ((rc = copy_image(ss, ss->img1, image1))) return rc;
     if ((rc = copy_image(ss, ss->img2s, image2s))) return rc;
     if ((rc = copy_image(ss, ss->img2m, image2m))) return rc;
@@ -2245,6 +2260,7 @@ int rtm_session_get_images_f64(rtm_session *ss, double *image1, double *image2s,
     if (!ss->o.accum_fp64) return fail(RTM_ERR_ARG, "session accumulates in fp32");
     CK(cudaSetDevice(ss->dev));
     CK(cudaStreamSynchronize(ss->stream));
+    if (int rc = wait_for_callers_work(ss)) return rc;
     size_t n = (size_t)ss->s.nx * ss->s.nz * 8;
     double *out[3] = {image1, image2s, illum};
     void *dev[3] = {ss->img1, ss->img2s, ss->illum};

@@ -25,9 +25,9 @@ class _DeviceArray:
 # images of several chunks (fp32, and fp64 narrowed on the way) and of less than a quarter of one
 @pytest.mark.gpu
 @pytest.mark.parametrize("nx,nz", [(600, 300), (160, 60)])
-@pytest.mark.parametrize("accum", [0, 1])
+@pytest.mark.parametrize("accum,f64", [(0, 0), (1, 0), (1, 1)])
 @pytest.mark.parametrize("blocking_stream", [False, True])
-def test_images_wait_for_work_on_the_default_stream(rtmlib, nx, nz, accum, blocking_stream):
+def test_images_wait_for_work_on_the_default_stream(rtmlib, nx, nz, accum, f64, blocking_stream):
     import torch
 
     G = rtmlib
@@ -48,9 +48,9 @@ def test_images_wait_for_work_on_the_default_stream(rtmlib, nx, nz, accum, block
         with torch.cuda.stream(st):
             torch.cuda._sleep(100_000_000)
             t.add_(1)
-        got = ss.images()["image1"].ravel()
+        got = (ss.images_f64() if f64 else ss.images())["image1"].ravel()
         torch.cuda.synchronize()
-        assert np.array_equal(got, want.astype(np.float32))
+        assert np.array_equal(got, want if f64 else want.astype(np.float32))
 
 
 RESET = """

@@ -24,7 +24,7 @@ FAKE = r"""
 
 // what the test sets and reads
 extern "C" {
-int alloc_left = -1, streams_left = -1, events_left = -1;   // successes left (-1: no limit)
+int alloc_left = -1, streams_left = -1;   // successes left (-1: no limit)
 int allocs = 0, stale = 0, live = 0;                        // calls that succeeded; uses of a lost handle
 unsigned long long context = 1;                             // a reset makes a new one
 }
@@ -37,7 +37,7 @@ namespace {
 std::recursive_mutex mu;
 thread_local int device = 0;
 thread_local cudaStream_t launch_stream;
-std::set<void *> handles;   // live streams, events and page-locked blocks
+std::set<void *> handles;   // live streams and page-locked blocks
 void *make(size_t n)
 {
     std::lock_guard<std::recursive_mutex> l(mu);
@@ -113,21 +113,6 @@ cudaError_t cudaStreamDestroy(cudaStream_t s)
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { return known(s) ? cudaSuccess : cudaErrorContextIsDestroyed; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { return known(s) && known(e) ? cudaSuccess : cudaErrorContextIsDestroyed; }
-cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned)
-{
-    if (!spend(events_left)) return cudaErrorMemoryAllocation;
-    *e = (cudaEvent_t)make(1);
-    return cudaSuccess;
-}
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return known(e) ? cudaSuccess : cudaErrorContextIsDestroyed; }
-cudaError_t cudaEventDestroy(cudaEvent_t e)
-{
-    if (!known(e)) return cudaErrorContextIsDestroyed;
-    std::lock_guard<std::recursive_mutex> l(mu);
-    handles.erase(e);
-    return cudaSuccess;
-}
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st)
 {
@@ -226,8 +211,8 @@ def _copies(L, seed=0):
         assert np.array_equal(g, f[:, :width])
 
 
-# no page-locked memory at all, for one lane, for three; the same for streams; no event
-@pytest.mark.parametrize("what", ["alloc_left", "streams_left", "events_left"])
+# no page-locked memory at all, for one lane, for three; the same for streams
+@pytest.mark.parametrize("what", ["alloc_left", "streams_left"])
 @pytest.mark.parametrize("left", [0, 1, 3])
 def test_copies_without_page_locked_memory_or_streams(rb, what, left):
     _var(rb, what).value = left
