@@ -6,6 +6,7 @@
 
 #include <algorithm>
 
+#include "rtm_div.cuh"
 #include "rtm_strip.cuh"
 #include "rtm_types.h"
 
@@ -404,19 +405,6 @@ __device__ __forceinline__ void st_row4(double *f, size_t id, const double (&v)[
     *(double2 *)(f + id + 2) = make_double2(v[2], v[3]);
 }
 
-// RN(a / b) for b > 0 given rb = RN(1 / b): two of Markstein's correction steps (exact residual by a
-// fused multiply-add; a faithful quotient so corrected is the rounded one), in the range where no
-// residual underflows; zero, which sends the library's division down its slow branch, is itself.
-__device__ __forceinline__ float div_by(float a, float b, float rb)
-{
-    if (fabsf(a) >= 1.0e-25f && fabsf(a) < 1.0e25f) {
-        float q = __fmul_rn(a, rb);
-        q = __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
-        return __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
-    }
-    return a == 0.0f ? a : __fdiv_rn(a, b);
-}
-
 template <int PAR, typename ACC>
 __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float dx, float dz, float dt)
 {
@@ -454,7 +442,7 @@ __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float
         ld_row4(S.b.vx, id, vx);
     }
     const float w0 = (float)(RTM_PI / 2.0 - (double)(0.5f * acosf(0.0f))), c0 = cosf(w0), s0 = sinf(w0);
-    const float rdx = __frcp_rn(dx), rdz = __frcp_rn(dz);
+    const Divisor ddx = divisor(dx), ddz = divisor(dz);
     ACC *g2p = (ACC *)S.gx[0], *g3p = (ACC *)S.gx[1], *g3tp = (ACC *)S.gx[2], *g4p = (ACC *)S.gx[3];
     ACC g2[4], g3[4], g3t[4], g4[4];
     ld_row4(g2p, id, g2);
@@ -502,10 +490,10 @@ __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float
         }
         // energy norm (kernel.cu:1486-1522)
         {
-            const float psx = div_by(0.5f * ((j < 3 ? ps[j + 1] : psr) - (j > 0 ? ps[j - 1] : psl)), dx, rdx);
-            const float psz = div_by(0.5f * (psd4[j] - psu4[j]), dz, rdz);
-            const float px = div_by(0.5f * ((j < 3 ? p[j + 1] : pr_) - (j > 0 ? p[j - 1] : pl_)), dx, rdx);
-            const float pz = div_by(0.5f * (pd4[j] - pu4[j]), dz, rdz);
+            const float psx = div_by(0.5f * ((j < 3 ? ps[j + 1] : psr) - (j > 0 ? ps[j - 1] : psl)), ddx);
+            const float psz = div_by(0.5f * (psd4[j] - psu4[j]), ddz);
+            const float px = div_by(0.5f * ((j < 3 ? p[j + 1] : pr_) - (j > 0 ? p[j - 1] : pl_)), ddx);
+            const float pz = div_by(0.5f * (pd4[j] - pu4[j]), ddz);
             const float dd = -(ps[j] - pspre[j]) * (p[j] - ppre[j]);
             const float e = dd == 0.0f ? dd : dd / (dt * dt * v2[j]);
             g4[j] += (ACC)(e + psx * px + psz * pz);
