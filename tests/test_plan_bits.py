@@ -120,3 +120,20 @@ def test_modelling_before_and_after_the_tuner_gives_the_same_gathers(rtmlib):
         ss.model()
         for k, g in enumerate(before):
             assert np.abs(g).max() > 0 and np.array_equal(ss.gather(k), g)
+
+
+# a batch of more than 400 MB of fields, whose tiles keep the order of the fields (smaller ones start with
+# the tiles that take longest), in merged and in separate launches
+@pytest.mark.gpu
+@pytest.mark.parametrize("heights", [(8, 8, 8, 8), (16, 16, 8, 8), (16, 16, 12, 8)])
+def test_large_batches_in_field_order(rtmlib, monkeypatch, heights):
+    G = rtmlib
+    nx, nz, shots = 350, 960, list(range(1, 27))   # 26 shots of 10 arrays of 416 x 1000 floats
+    v, rho = _models(nz, nx, 26)
+    out = []
+    for env in ({"RTM_B200_KERNELS": "scalar", "RTM_B200_TUNE": "0"}, _heights(*heights)):
+        with monkeypatch.context() as m:
+            for k, x in env.items():
+                m.setenv(k, x)
+            out.append(G.migrate(_survey(G, nx=nx, nz=nz, nt=40), G.RunOptions(), shots, v, rho))
+    _same(out[1], out[0])
