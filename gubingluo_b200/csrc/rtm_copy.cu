@@ -141,7 +141,8 @@ int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, siz
     std::atomic<int> err{(int)cudaSuccess};
     const unsigned long long ctx = context_id();   // (the library runs in the device's primary context only)
     const int nt = (int)std::min<size_t>(kLanes, n);
-#pragma omp parallel num_threads(nt)
+    const bool team = host_team();
+#pragma omp parallel num_threads(nt) if (team)
     {
         Lane l;
         cudaError_t e = cudaSetDevice(dev);

@@ -2,6 +2,9 @@
 // coefficient table, SU/SEG-Y/image files and the parameter file.  Each function states
 // the reference routine whose behaviour (including its float/double evaluation order and
 // integer truncations) it reproduces.
+#include <unistd.h>
+
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -202,6 +205,17 @@ void pml_smooth(float *vp, int nx, int nz, int npml)
     }
 }
 
+// False in a process that was forked after its parent ran a team (for smoothing, or for read-back): it has the
+// OpenMP library's records of the team's threads but not the threads, and a team of its own would wait for
+// them without end.  Teams are therefore run `if (host_team())`, else by the calling thread alone.
+bool host_team()
+{
+    static std::atomic<int> first{0};   // the process that ran a team first
+    int seen = 0;
+    const int me = (int)getpid();
+    return first.compare_exchange_strong(seen, me) || seen == me;
+}
+
 // velsmooth1d (Velocity_function.cpp:199-313): 2-D Gaussian of half-width nsp and
 // sigma = nsp/3 over an edge-replicated extension; weights and sums in double, each
 // output cell summed in the reference's (row, column) order.
@@ -227,7 +241,8 @@ void gauss_smooth(float *vp, int n1, int n2, int nsp)
             norm += std::exp(-(d1 * d1 + d2 * d2) / (2.0 * nsp / 3.0 * nsp / 3.0));
         }
     std::vector<float> out((size_t)n1 * n2);
-#pragma omp parallel for schedule(dynamic, 4)
+    const bool team = host_team();
+#pragma omp parallel for schedule(dynamic, 4) if (team)
     for (int i1 = 0; i1 < n1; i1++)
         for (int i2 = 0; i2 < n2; i2++) {
             double acc = 0;

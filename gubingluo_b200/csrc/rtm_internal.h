@@ -25,6 +25,8 @@ void interp_model(const float *vp0, float *vp, int nx0, int nz0, int nx, int lx,
 void get_constant(const float *vp, float fdom, float dx0, float dz0, int nx0, int nz0, int nt0, float dt0,
                   float *dx, float *dz, int *nx, int *nz, int *nt, float *dt, int *lx, int *lz, float *vpmin,
                   float *vpmax);
+// Whether this process may run a team of OpenMP threads (rtm_host.cpp).
+bool host_team();
 // Device rows into packed host rows (rtm_copy.cu); narrow: doubles into floats.
 int copy_out(void *dst, const void *src, size_t src_pitch, size_t row_bytes, size_t rows, bool narrow = false);
 
