@@ -1181,7 +1181,7 @@ static int batch_setup(rtm_session *ss, int k0, int n, BatchRun &br)
     return RTM_OK;
 }
 
-// The kernel forms as bits (1: four columns per thread) of vel, vel_recon, pres, pres_recon.
+// The kernel forms as bits (1: pipelined) of vel, vel_recon, pres, pres_recon.
 static int form_bits(const rtm_session *ss)
 {
     return (ss->vec[0] ? 1 : 0) | (ss->vec[1] ? 2 : 0) | (ss->vec[2] ? 4 : 0) | (ss->vec[3] ? 8 : 0);
@@ -1328,8 +1328,8 @@ static int persistent_pass(rtm_session *ss, BatchRun &br, int dir, int nsteps, b
 }
 
 // Source pass (rtm_model.cu:322-346): nsteps forward steps with the source added; strips
-// saved after every step when `save` (one small copy kernel, so the stencil kernels carry no
-// strip logic); the gather recorded when `record` (mode 0 fuses the reference's separate
+// saved in every step when `save` (by the tiles that hold their cells in the pipelined form, else by
+// a small copy kernel after the step); the gather recorded when `record` (mode 0 fuses the reference's separate
 // modelling pass, rtm_model.cu:266-290, which is the same computation in the same model,
 // into this pass).
 static int batch_forward(rtm_session *ss, BatchRun &br, int nsteps, bool save, bool record)

@@ -1,5 +1,5 @@
-// rtm_stencil_common.cuh — device helpers shared by the stencil kernels (rtm_stencil.cu:
-// one column per thread; rtm_stencil_v.cu: four columns by U rows per thread): tile staging
+// rtm_stencil_common.cuh — device helpers shared by the stencil kernels (rtm_pipe.cu: the pipelined
+// form; rtm_stencil.cu: one column per thread; rtm_step.cu: whole steps): tile staging
 // by the tensor memory accelerator with bounded waits, strip indexing, and the update
 // formulas, rounded operation by operation so that every kernel form gives the same bits.
 #pragma once
@@ -54,12 +54,6 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-// Before an mbarrier's memory is initialised again (a block that stages one tile after
-// another), the old object is invalidated; every wait on it has completed by then.
-__device__ __forceinline__ void mbar_inval(unsigned long long *bar)
-{
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_expect(unsigned long long *bar, unsigned bytes)
 {
@@ -186,7 +180,8 @@ __device__ __forceinline__ int strip_row_tb(int z, int npml, int first, int nxi)
 // Interior pressure update p - (dxs + dzs) and the cross-correlation terms, shared by the
 // general and the interior-tile forms of the pressure kernel so that both give the same
 // bits: the sum and the difference are rounded separately (no fused multiply-add), as the
-// reference's host-order arithmetic and the oracle have them.
+// reference's host-order arithmetic and the oracle have them (but for the source pass's interior tiles
+// with the other imaging conditions, StepArgs::fuse).
 __device__ __forceinline__ float p_interior(float p0, float dxs, float dzs) { return __fsub_rn(p0, __fadd_rn(dxs, dzs)); }
 template <typename ACC>
 __device__ __forceinline__ ACC image_g1(ACC og1, float ps, float pn) { return og1 + (ACC)ps * (ACC)pn; }

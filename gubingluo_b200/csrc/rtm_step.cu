@@ -1,7 +1,7 @@
 // rtm_step.cu — one whole time step (velocity and pressure) of one wavefield per launch
 // (sm_100a).
 //
-// The split kernels (rtm_stencil.cu, rtm_stencil_v.cu) update the velocities of a step in
+// The split kernels (rtm_pipe.cu, rtm_stencil.cu) update the velocities of a step in
 // one launch and the pressure in the next, so p, vx and vz cross HBM twice per step: 44 bytes
 // per cell-update.  Here one launch does both, reading p, vx, vz, 1/rho and kappa once and
 // writing p, vx and vz once (32 bytes).  The pressure update at a cell needs the new vx of the

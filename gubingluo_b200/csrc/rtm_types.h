@@ -48,7 +48,8 @@
 // What one launch of the stencil kernels updates.
 enum RtmWaveMode {
     RTM_WAVE_FWD = 0,        // forward propagation, full grid (modelling and source pass;
-                             // the source pass saves its strips with k_strip_save)
+                             // the source pass's strips are saved by the pipelined kernels
+                             // themselves, else by k_strip_save)
     RTM_WAVE_RECEIVER = 2,   // receiver back-propagation (+ injection; imaging in the p update)
     RTM_WAVE_RECON = 3       // source-wavefield reconstruction (interior + restored strips)
 };

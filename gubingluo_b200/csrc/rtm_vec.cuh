@@ -1,5 +1,5 @@
 // rtm_vec.cuh — 16-byte-word helpers of the kernels that give each thread four adjacent
-// columns (rtm_stencil_v.cu, rtm_step.cu): shared and global float4 accesses, x- and
+// columns (rtm_pipe.cu, rtm_step.cu): shared and global float4 accesses, x- and
 // z-derivative sums of four columns from staged rows, accumulator words.
 #pragma once
 #include <type_traits>
@@ -142,11 +142,5 @@ __device__ __forceinline__ void dz4(const float *col, float (&s)[U][4], C coef)
     }
 #endif
 }
-
-// Resident blocks per SM that leave each of `threads` threads `regs` registers (the launch
-// bounds of the kernels below: 80 registers, 128 for the receiver pressure update with its
-// imaging operands; measured with -Xptxas -v, no spills at 16-row tiles in fp32 but 24 bytes
-// in the receiver pressure update).
-constexpr int min_blocks(int threads, int regs) { return 65536 / (threads * regs) > 0 ? 65536 / (threads * regs) : 1; }
 
 }  // namespace
