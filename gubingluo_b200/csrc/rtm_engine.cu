@@ -532,7 +532,9 @@ static int open_session(rtm_session *ss, const float *vp, const float *rho, cons
             ss->tune = false;
             ss->bz_vel = 32;
             ss->bz_vel_recon = 16;
+            // (the other imaging conditions run per-step launches all the same, at their own height)
             ss->bz_pres = ss->bz_pres_recon = 16;
+            if (o.extra_images) ss->bz_pres = extra_pres_height(ss);
             for (bool &v : ss->vec) v = false;
         }
         if (o.extra_images < 0 || o.extra_images > 2) return fail(RTM_ERR_ARG, "extra_images must be 0, 1 or 2");

@@ -75,7 +75,8 @@ def test_batching_and_resume_give_one_set_of_bits_on_wide_grids(rtmlib, monkeypa
     want = _run(G, monkeypatch, PLANS["no tuner"], options)
     for batch in (0, 1, 2):
         _same(_run(G, monkeypatch, {}, dict(options, batch=batch)), want, keys)
-    _same(_run(G, monkeypatch, {"RTM_B200_TUNE": "0", "RTM_B200_KERNELS": "scalar"}, options), want, keys)
+    for env in ({"RTM_B200_TUNE": "0", "RTM_B200_KERNELS": "scalar"}, {"RTM_B200_PERSIST": "1"}):
+        _same(_run(G, monkeypatch, env, options), want, keys)
     v, rho = _models(NZ, NX, 3)
     path = str(tmp_path / "run.ckpt")
     with G.Session(_survey(G), G.RunOptions(batch=2, **options), SHOTS, v, rho) as a:
