@@ -62,7 +62,6 @@ __device__ __forceinline__ float2 both(float c) { return make_float2(c, c); }
 // -1: every sum below is written as the difference of a negated product.
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, both(-1.f), a); }
 
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
 // Four adjacent columns as two pairs.
 struct P4 {
@@ -564,11 +563,14 @@ __device__ __forceinline__ void pres_compute(const StepArgs &a, const StageMeta<
             if (MODE == 2 && !staged && u + 1 < U) load_img(u + 1);
             const P4 dx = dx_sum<11, 12>(rowbase + u * WW, cx);
             const P4 kk = p4(lds4(op + u * BX)), p0 = p4(lds4(op + (BZ + u) * BX));
-            const P4 ax = mul(dx, dtx), maz = mul(mul(dz[u], mdtz), kk);
-            P4 d;
-            if (MODE == 0 && a.fuse) d = {__ffma2_rn(ax.a, kk.a, neg2(maz.a)), __ffma2_rn(ax.b, kk.b, neg2(maz.b))};
-            else d = sub(mul(ax, kk), maz);
-            const float4 pn = q4(sub(p0, d));
+            const P4 maz = mul(mul(dz[u], mdtz), kk);
+            float4 pn;
+            if (MODE == 0 && a.fuse) {   // p0 - fma(ax, kk, az) as p0 + fma(-ax, kk, -az)
+                const P4 nax = mul(dx, -a.dtx);
+                pn = q4({__fadd2_rn(p0.a, __ffma2_rn(nax.a, kk.a, maz.a)), __fadd2_rn(p0.b, __ffma2_rn(nax.b, kk.b, maz.b))});
+            } else {
+                pn = q4(sub(p0, sub(mul(mul(dx, dtx), kk), maz)));
+            }
             st4(&pp[id0 + u * pitch], pn);
             if (MODE == 2) image(u, pn);
         }
