@@ -405,7 +405,8 @@ __device__ __forceinline__ void st_row4(double *f, size_t id, const double (&v)[
     *(double2 *)(f + id + 2) = make_double2(v[2], v[3]);
 }
 
-template <int PAR, typename ACC>
+// FAR: a grid spacing that div_by does not take.
+template <int PAR, typename ACC, bool FAR>
 __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float dx, float dz, float dt)
 {
     const ShotDev &S = shots[blockIdx.z];
@@ -442,7 +443,8 @@ __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float
         ld_row4(S.b.vx, id, vx);
     }
     const float w0 = (float)(RTM_PI / 2.0 - (double)(0.5f * acosf(0.0f))), c0 = cosf(w0), s0 = sinf(w0);
-    const Divisor ddx = divisor(dx), ddz = divisor(dz);
+    const float rdx = __frcp_rn(dx), rdz = __frcp_rn(dz);
+    const auto over = [](float a, float b, float rb) { return FAR ? __fdiv_rn(a, b) : div_by(a, b, rb); };
     ACC *g2p = (ACC *)S.gx[0], *g3p = (ACC *)S.gx[1], *g3tp = (ACC *)S.gx[2], *g4p = (ACC *)S.gx[3];
     ACC g2[4], g3[4], g3t[4], g4[4];
     ld_row4(g2p, id, g2);
@@ -490,10 +492,10 @@ __global__ void __launch_bounds__(256) k_image_extra(const ShotDev *shots, float
         }
         // energy norm (kernel.cu:1486-1522)
         {
-            const float psx = div_by(0.5f * ((j < 3 ? ps[j + 1] : psr) - (j > 0 ? ps[j - 1] : psl)), ddx);
-            const float psz = div_by(0.5f * (psd4[j] - psu4[j]), ddz);
-            const float px = div_by(0.5f * ((j < 3 ? p[j + 1] : pr_) - (j > 0 ? p[j - 1] : pl_)), ddx);
-            const float pz = div_by(0.5f * (pd4[j] - pu4[j]), ddz);
+            const float psx = over(0.5f * ((j < 3 ? ps[j + 1] : psr) - (j > 0 ? ps[j - 1] : psl)), dx, rdx);
+            const float psz = over(0.5f * (psd4[j] - psu4[j]), dz, rdz);
+            const float px = over(0.5f * ((j < 3 ? p[j + 1] : pr_) - (j > 0 ? p[j - 1] : pl_)), dx, rdx);
+            const float pz = over(0.5f * (pd4[j] - pu4[j]), dz, rdz);
             const float dd = -(ps[j] - pspre[j]) * (p[j] - ppre[j]);
             const float e = dd == 0.0f ? dd : dd / (dt * dt * v2[j]);
             g4[j] += (ACC)(e + psx * px + psz * pz);
@@ -604,12 +606,13 @@ void launch_image_extra(const ShotDev *shots, int nshots, int max_nxi, int max_n
 {
     // (up to three columns before the interior's first belong to its first word)
     dim3 grid((max_nxi + 3 + 127) / 128, (max_nzi + 7) / 8, nshots), block(32, 8);
-    if (parity) {
-        if (fp64) k_image_extra<1, double><<<grid, block, 0, s>>>(shots, dx, dz, dt);
-        else k_image_extra<1, float><<<grid, block, 0, s>>>(shots, dx, dz, dt);
+    const auto go = [&](auto kernel) { kernel<<<grid, block, 0, s>>>(shots, dx, dz, dt); };
+    if (!div_by_takes(dx) || !div_by_takes(dz)) {
+        if (parity) fp64 ? go(k_image_extra<1, double, true>) : go(k_image_extra<1, float, true>);
+        else fp64 ? go(k_image_extra<0, double, true>) : go(k_image_extra<0, float, true>);
     } else {
-        if (fp64) k_image_extra<0, double><<<grid, block, 0, s>>>(shots, dx, dz, dt);
-        else k_image_extra<0, float><<<grid, block, 0, s>>>(shots, dx, dz, dt);
+        if (parity) fp64 ? go(k_image_extra<1, double, false>) : go(k_image_extra<1, float, false>);
+        else fp64 ? go(k_image_extra<0, double, false>) : go(k_image_extra<0, float, false>);
     }
 }
 void launch_finalize_extra(const void *fs, int nshots, int nx, int nz, int fp64, void *const img[7], cudaStream_t s)
