@@ -207,7 +207,8 @@ int rtm_session_get_gather(rtm_session *ss, int k, float *gather);
  * for the vpmax of the shot's model window): ddx [nxpad], ddz [nzpad], ddxvx [nxpad-1],
  * ddzvz [nzpad-1]; any pointer may be NULL.  For parity tests. */
 int rtm_session_get_pml(rtm_session *ss, int k, float *ddx, float *ddz, float *ddxvx, float *ddzvz);
-/* Copy the stacked images (nz*nx each; any pointer may be NULL). */
+/* Copy the stacked images (nz*nx each; any pointer may be NULL), after work that the caller queued on
+ * them (rtm_session_image_ptrs) in the default stream or in one that synchronises with it. */
 int rtm_session_get_images(rtm_session *ss, float *image1, float *image2s, float *image2m,
                            float *illum);
 int rtm_session_get_images_f64(rtm_session *ss, double *image1, double *image2s, double *illum);
