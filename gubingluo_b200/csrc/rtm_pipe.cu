@@ -32,7 +32,7 @@
 // What bounds it: 64 shots of 1801x451, us a launch at 1965 MHz (one tile per block before; each field
 // read and written once at 6.46 TB/s): receiver velocity 192 (248; 191), forward velocity with its strips
 // 210 (251 + 28; 193), receiver pressure and imaging 317 (347; 302): the memory's rate at that clock.
-// Forward pressure 258 (281; 187): latency of shared-memory reads and instructions.  Reconstruction 171
+// Forward pressure 252 (281; 187): latency of shared-memory reads and instructions.  Reconstruction 171
 // and 140 (191, 176; 144, 120): the tiles with strips.  A long run is power-capped to 1690-1890 MHz, and
 // there the first three read 0.88-0.94 of the memory's rate and gain 10% from 16% more clock: the SMs'
 // side (shared-memory reads and their latency) bounds them as much as the memory.  One shot of 401x201: 4.6 us a launch (7 launches of 7 us a
