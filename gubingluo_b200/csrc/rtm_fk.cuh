@@ -24,9 +24,9 @@
 // the middle one the last levels, the product with the spectrum and the first levels back, the first
 // reads its input and the last writes its result: 6 passes at M = 8192 (one level a pass, one trace a
 // transform and the phases worked out in place took 16).  A shot in a session with its upload, ms,
-// cuFFT / one level a pass / now: 241 traces x 2000 samples, lx = 2, 0.35 / 0.39 / 0.25; x 4000 0.65 / 0.83 / 0.52;
-// 400 x 4000, lx = 4, 1.43 / 2.23 / 1.26; 1024 x 4096, lx = 4, 3.7 / 5.9 / 3.1; 400 x 700, lx = 2, 0.19 / 0.30 / 0.19;
-// cuFFT is ahead for few long traces, where a launch has fewer blocks than SMs: 60 x 4000 0.17 / - / 0.21.
+// cuFFT / one level a pass / now: 241 traces x 2000 samples, lx = 2, 0.35 / 0.39 / 0.25; x 4000 0.65 / 0.83 / 0.50;
+// 400 x 4000, lx = 4, 1.43 / 2.23 / 1.25; 1024 x 4096, lx = 4, 3.7 / 5.9 / 2.9; 400 x 700, lx = 2, 0.19 / 0.30 / 0.19;
+// cuFFT is ahead for few long traces, where a launch has fewer blocks than SMs: 60 x 4000 0.17 / - / 0.20.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -357,20 +357,32 @@ __device__ __forceinline__ float cabs_f(double re, double im)
     return sqrtf(__double2float_rn(__dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im))));
 }
 
-// Space transforms of time frequency kt, block (kt, part): part lx the fold Z (kept below nf) and the
-// max |Z| over all frequencies (non-negative floats order like their bits); part r the frequencies lx k + r
-// of S below nf, and K, its part 0 at every lx-th frequency.
+// Space transforms, one per block: first the folds Z of every time frequency kt (kept below nf) and the
+// max |Z| over all of them (non-negative floats order like their bits); then the frequencies lx k + r of S for
+// kt below nf; then K's rows, part 0 at every lx-th frequency, that are not below nf (those that are
+// come with S).
+__host__ __device__ inline int space_blocks(int nh, int nf, int lx) { return nh + nf * lx + nf - (nf + lx - 1) / lx; }
 __global__ void __launch_bounds__(512) k_fk_space(const FkArgs a)
 {
     extern __shared__ double2 x[];
-    const int kt = blockIdx.x, r = blockIdx.y, it = kt / a.lx;
-    const bool fold = r == a.lx, isk = r == 0 && it * a.lx == kt && it < a.nf;
-    if (!fold && kt >= a.nf && !isk) return;
+    int kt = blockIdx.x, r = 0;
+    const bool fold = kt < a.nh;
+    if (!fold) {
+        kt -= a.nh;
+        if (kt < a.nf * a.lx) {
+            r = kt % a.lx;
+            kt /= a.lx;
+        } else {
+            kt = (kt - a.nf * a.lx + (a.nf + a.lx - 1) / a.lx) * a.lx;
+        }
+    }
+    const int it = kt / a.lx;
+    const bool isk = r == 0 && it * a.lx == kt && it < a.nf;
     const int np = (a.nx0 + 1) / 2;
     const double2 *row = a.A + (size_t)kt * np, *neg = a.A + (size_t)(kt ? a.Nt - kt : 0) * np;
     float mx = 0.0f;
     chirp_dft(
-        x, a.nx0, fold ? 0 : r, a.px, a.cx, a.tw, a.mt, a.nx0,
+        x, a.nx0, r, a.px, a.cx, a.tw, a.mt, a.nx0,
         [&](int i) {
             const long long t = fold ? (long long)i * a.lx : i;
             return t < a.nx0 ? trace_at(row, neg, (int)t) : make_double2(0.0, 0.0);

@@ -437,7 +437,7 @@ static int interp_run(InterpPlan &p, float *out, float dt, float dt0, int mirror
         CKI(cudaMemsetAsync(p.zmax, 0, sizeof(unsigned), st));
         const int mT = fk::pow2_for(sh.nt0), mx = fk::pow2_for(sh.nx0), mX = fk::pow2_for(sh.Nx);
         fk::k_fk_time<<<dim3((sh.nx0 + 1) / 2, sh.lx), fk::threads(mT), fk::smem_bytes(mT), st>>>(a);
-        fk::k_fk_space<<<dim3(a.nh, sh.lx + 1), fk::threads(mx), fk::smem_bytes(mx), st>>>(a);
+        fk::k_fk_space<<<fk::space_blocks(a.nh, a.nf, a.lx), fk::threads(mx), fk::smem_bytes(mx), st>>>(a);
         fk::k_fk_filter<<<sh.nf, fk::threads(mX), fk::smem_bytes(mX), st>>>(a);
         fk::k_fk_back<<<(sh.nx + 1) / 2, fk::threads(mT), fk::smem_bytes(mT), st>>>(a);
         if (launches) *launches += 4;

@@ -178,7 +178,8 @@ def test_a_result_beyond_the_device_memory_is_refused(rtmlib):
 # 1e5 in size, and lengths in x whose power of two (16 to 8192 points) takes every order of passes
 @pytest.mark.gpu
 @pytest.mark.parametrize("nx0,nt0,lx", [(2, 9, 2), (3, 40, 2), (4, 41, 3), (5, 8, 4), (17, 30, 3), (33, 60, 5),
-                                        (65, 130, 2), (129, 20, 3), (250, 30, 4), (512, 21, 4), (1300, 12, 3)])
+                                        (65, 130, 2), (129, 20, 3), (250, 30, 4), (512, 21, 4), (1300, 12, 3), (2, 10, 300),
+                                        (3, 12, 64)])
 @pytest.mark.parametrize("mirror", [0, 1])
 def test_pairs_of_traces_and_every_order_of_passes(rtmlib, nx0, nt0, lx, mirror):
     from test_fk import _fk
